@@ -207,15 +207,15 @@ int launch_seg(const CUtensorMap* maps, const SegArgs& a, int groups, cudaStream
     return launch_seg_rr<METHOD, CYCLIC, 0>(maps, a, groups, st);
 }
 
-// 3-D view [nseg][TILE_MT][n_sys] of an [n_row x n_sys] FP64 array; boxes of
-// tile_rps(elem, na) rows of `nsc` consecutive sub-segments for `sys` systems
-// (na: arrays of the ring the boxes go to).
+// 3-D view [nseg][mt][n_sys] of an [n_row x n_sys] FP64 array (mt rows a
+// sub-segment); boxes of tile_rps(elem, na) rows of `nsc` consecutive
+// sub-segments for `sys` systems (na: arrays of the ring the boxes go to).
 inline bool make_tile_map(CUtensorMap* map, const void* ptr, int n_sys, int nseg, int sys,
-                          int nsc, int elem = 8, int na = 4) {
+                          int nsc, int elem = 8, int na = 4, int mt = TILE_MT) {
     auto fn = encode_fn();
     if (!fn) return false;
-    cuuint64_t dims[3] = {(cuuint64_t)n_sys, (cuuint64_t)TILE_MT, (cuuint64_t)nseg};
-    cuuint64_t strides[2] = {(cuuint64_t)n_sys * elem, (cuuint64_t)n_sys * TILE_MT * elem};
+    cuuint64_t dims[3] = {(cuuint64_t)n_sys, (cuuint64_t)mt, (cuuint64_t)nseg};
+    cuuint64_t strides[2] = {(cuuint64_t)n_sys * elem, (cuuint64_t)n_sys * mt * elem};
     cuuint32_t box[3] = {(cuuint32_t)sys, (cuuint32_t)tile_rps(elem, na), (cuuint32_t)nsc};
     cuuint32_t estr[3] = {1, 1, 1};
     const CUtensorMapDataType dt =
@@ -385,30 +385,43 @@ int launch_tile_plan(const TilePlan& pl, const CUtensorMap* maps, const TileArgs
     }
 }
 
-// BTDMA_TILE_AUTO's choice between the kernels for a shape both take, from
-// B200 measurements (262144 x 512, 524288 x 256, 1048576 x 128; ms):
-//   FP32 storage  narrow 1.03 / 0.81 / 0.83   wide 0.82 / 0.73 / 0.72
-//   FP64          narrow 1.06 / 0.97 / 0.96   wide 1.03 / 1.02 / 1.01
-// The narrow kernel reads 64-byte row pieces for FP32 at 512 rows and 128-byte
-// pieces elsewhere; the wide kernel's extra pass over half the rows pays off
-// for FP32 storage everywhere and for FP64 above 16 sub-segments only.
-inline bool wide_by_default(int n_row, int elem) {
-    return elem == 4 || n_row / TILE_MT > 16;
-}
-
-// Plan of the wide-box kernel (k_tile_wide.cuh): sys == 0 when the shape does
-// not take it.
-inline TilePlan tile_wide_plan(int n_row, bool cyclic, int elem) {
+// Plan of the wide kernel (k_tile_wide.cuh), nseg in 32-row sub-segments: sys ==
+// 0 when the shape does not take it, or (not forced) the narrow one is faster.
+//
+// The widest box, so that a CTA has 512 threads, is the fastest wherever it
+// leaves enough groups: B200, us, narrow / wide by systems per CTA,
+//   262144 x 512 FP64   1098 / 817 (32 systems), 1169 (16)
+//   262144 x 256 FP64    571 / 413 (64), 620 (32), 683 (16)
+//   262144 x 128 FP64    254 / 210 (128), 246 (64), 350 (32)
+//   1048576 x 64 FP64    494 / 407 (256), 552 (128), 654 (64)
+//   262144 x 512 FP32   1067 / 523 (32); 262144 x 256 FP32 430 / 258 (64)
+// Few groups: with at most half the SMs busy, half the systems per CTA are
+// faster (4096 x 256 FP64: 14.8 at 64 groups, 11.8 at 128; 2048 x 512: 14.8 at
+// 64, 11.7 at 128) down to 256 threads; below that the narrow kernel's shorter
+// sub-segments win (2048 x 128: 8.3 / 9.1; FP32 2048 x 128: 5.8 / 7.2).
+inline TilePlan tile_wide_plan(int n_row, int n_sys, bool cyclic, int elem, bool forced) {
     TilePlan pl;
-    if (n_row % TILE_MT != 0) return pl;
-    const int nseg = n_row / TILE_MT;
-    if (nseg < 8 || nseg > 32 || nseg % 2 != 0) return pl;
+    if (n_row % WIDE_M != 0) return pl;
+    const int nseg = n_row / WIDE_M;
+    if (nseg < (forced ? 4 : 2) || nseg > 16) return pl;
     if (cyclic && (nseg & (nseg - 1)) != 0) return pl;
-    const int h = nseg / 2;
-    const int sys = h > 8 ? 32 : (h > 4 ? 64 : 128);
+    int sys = nseg > 8 ? 32 : (nseg > 4 ? 64 : (nseg > 2 ? 128 : 256));
+    if (!forced) {
+        const int min_sys = nseg == 16 ? 16 : 32;  // whole warps
+        while (2 * ((n_sys + sys - 1) / sys) <= num_sms()) {
+            if (sys / 2 * nseg < 256 || sys == min_sys) {
+                if (sys == 16) break;  // 512 rows: as fast as the narrow kernel
+                return pl;
+            }
+            sys /= 2;
+        }
+    }
     int nst = TILE_MAX_NST;
-    while (nst >= 3 && tile_wide_smem_bytes(sys, nseg, nst, elem) > (size_t)max_smem_optin())
-        --nst;
+    // an equal share of the SM per resident CTA (128 registers a thread)
+    const int per_sm = std::max(1, TILE_MAX_THREADS / (sys * nseg));
+    const size_t cap = std::min((size_t)max_smem_optin(),
+                                (size_t)max_smem_per_sm() / per_sm - 1024);
+    while (nst >= 3 && tile_wide_smem_bytes(sys, nseg, nst, elem) > cap) --nst;
     if (nst < 3) return pl;
     pl.sys = sys;
     pl.cl = 1;
@@ -426,9 +439,11 @@ int launch_tile_wide(const CUtensorMap* maps, const TileArgs& a, cudaStream_t st
                                 max_smem_optin()));
         attr_done = true;
     }
-    const int threads = SYS * (a.nseg / 2);
+    const int threads = SYS * a.nseg;
     const size_t smem = tile_wide_smem_bytes(SYS, a.nseg, a.nst, (int)sizeof(TIN));
-    const int grid = std::min(num_sms(), a.n_groups);
+    int nb = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, threads, smem));
+    const int grid = std::min(num_sms() * std::max(1, nb), a.n_groups);
     kern<<<grid, threads, smem, st>>>(maps[0], maps[1], maps[2], maps[3], a);
     CK(cudaGetLastError());
     return BTDMA_OK;
@@ -443,6 +458,10 @@ int launch_tile_wide_plan(const TilePlan& pl, const CUtensorMap* maps, const Til
         case 128: return launch_tile_wide<64, false, TIN, FILT>(maps, a, st);
         case 129: return launch_tile_wide<64, true, TIN, FILT>(maps, a, st);
         case 65: return launch_tile_wide<32, true, TIN, FILT>(maps, a, st);
+        case 512: return launch_tile_wide<256, false, TIN, FILT>(maps, a, st);
+        case 513: return launch_tile_wide<256, true, TIN, FILT>(maps, a, st);
+        case 32: return launch_tile_wide<16, false, TIN, FILT>(maps, a, st);
+        case 33: return launch_tile_wide<16, true, TIN, FILT>(maps, a, st);
         default: return launch_tile_wide<32, false, TIN, FILT>(maps, a, st);
     }
 }
@@ -467,8 +486,8 @@ int try_tile(const TIN* A, const TIN* B, const TIN* C, const TIN* D, double* X, 
     bool wide = false;
     TilePlan pl;
     if (shape != BTDMA_TILE_NARROW && sizeof(TC) == 8 && !accumulate) {
-        pl = tile_wide_plan(n_row, cyclic, elem);
-        wide = pl.sys != 0 && (shape == BTDMA_TILE_WIDE || wide_by_default(n_row, elem));
+        pl = tile_wide_plan(n_row, n_sys, cyclic, elem, shape == BTDMA_TILE_WIDE);
+        wide = pl.sys != 0 && filt_r % 2 == 0;  // whole 32-row sub-segments
     }
     if (!wide) {
         pl = tile_plan(n_row, cyclic, elem);
@@ -481,14 +500,15 @@ int try_tile(const TIN* A, const TIN* B, const TIN* C, const TIN* D, double* X, 
     if (!(tma_ok_elem(A, n_sys, elem) && tma_ok_elem(B, n_sys, elem) &&
           tma_ok_elem(C, n_sys, elem) && tma_ok_elem(D, n_sys, elem)))
         return 0;
-    // sub-segments per TMA box: the CTA's share (narrow), or half a system (wide)
-    const int nsc = wide ? pl.nseg / 2 : pl.nseg / pl.cl;
+    const int nsc = pl.nseg / pl.cl;  // sub-segments per TMA box: the CTA's share
+    const int mt = wide ? WIDE_M : TILE_MT;
     CUtensorMap maps[4];
-    if (!(make_tile_map(&maps[0], A, n_sys, pl.nseg, pl.sys, nsc, elem) &&
-          make_tile_map(&maps[1], B, n_sys, pl.nseg, pl.sys, nsc, elem) &&
-          make_tile_map(&maps[2], C, n_sys, pl.nseg, pl.sys, nsc, elem) &&
-          make_tile_map(&maps[3], D, n_sys, pl.nseg, pl.sys, nsc, elem)))
+    if (!(make_tile_map(&maps[0], A, n_sys, pl.nseg, pl.sys, nsc, elem, 4, mt) &&
+          make_tile_map(&maps[1], B, n_sys, pl.nseg, pl.sys, nsc, elem, 4, mt) &&
+          make_tile_map(&maps[2], C, n_sys, pl.nseg, pl.sys, nsc, elem, 4, mt) &&
+          make_tile_map(&maps[3], D, n_sys, pl.nseg, pl.sys, nsc, elem, 4, mt)))
         return 0;
+    if (wide) filt_r /= 2;  // Filtered segments in 32-row sub-segments
     TileArgs a = {};
     a.X = X;
     a.n_sys = n_sys;

@@ -1,35 +1,37 @@
-// Wide-box variant of the register-tiled segmented solve (k_tile.cuh): twice the
-// systems per CTA, so every row of a TMA box is twice as wide in HBM.
+// Wide variant of the register-tiled segmented solve (k_tile.cuh): sub-segments
+// of 32 rows, whose elimination state is held half in registers and half in
+// tensor memory, so a CTA takes twice the systems and every row of a TMA box is
+// twice as wide in HBM.
 //
 // Why: the DRAM serves a stream of row pieces (SYS x element bytes, rows a full
 // row of the batch apart) at a rate that grows with the piece width: 64-byte
 // pieces reach about half the bandwidth of 128-byte ones, 128-byte pieces about
-// three quarters of 256-byte ones.  The tiled kernel keeps the elimination state
-// of all its rows in registers, which caps it at 16 systems of 512 rows per SM
-// (64-byte pieces for FP32 storage).  This kernel takes SYS = 512 / (NSEG / 2)
-// systems (32 at 512 rows, 64 at 256) and holds only half of every group's state:
+// three quarters of 256-byte ones.  The tiled kernel keeps the state of all its
+// rows in registers (24 bytes a row), which caps it at 16 systems of 512 rows
+// per SM.  The SM's 256 KB of tensor memory is per-thread storage too: a warp
+// reads and writes its own quarter of the lanes (tcgen05.st / tcgen05.ld, 32
+// lanes x 32-bit columns), one 96-column slice per warp holding 16 rows' alpha,
+// gamma and delta of each thread.  With it a CTA takes 32 systems of 512 rows.
 //
-//   A0  sub-segments 0 .. H-1 (H = NSEG / 2), thread (s, q) = system s,
-//       sub-segment q: the forward pass of k_tile.cuh reduced to its running
-//       scalars; only the two reduced rows are kept.
-//   A1  sub-segments H .. NSEG-1, thread (s, q) takes H + q: the same pass with
-//       the per-row state in registers, as in k_tile.cuh.
-//   reduced system: one warp-shuffle solve per system (reduced_solve_shfl).
-//   B1  back substitution of A1's sub-segments from registers.
-//   B0  the rows of A0 are loaded again (read earlier in the same group, mostly
-//       still in L2), the forward pass is repeated with its state in registers,
-//       and the back substitution follows.
+//   forward   thread (s, q) = system s, rows 32 q .. 32 q + 31: the pass of
+//             k_tile.cuh over 32 rows; after row 15 the state of rows 0..15
+//             moves to tensor memory, rows 16..31 stay in registers.
+//   reduced   one system per group of W lanes (reduced_solve_shfl), half as
+//             many rows as with 16-row sub-segments.
+//   back      rows 31..16 from registers, then rows 15..0 from tensor memory.
 //
-// The ring (as in k_tile.cuh: full/empty mbarriers per stage, refills issued by
-// a rotating producer warp; here with unhinted polls) carries 3 * SPG stages
-// per group: A0, A1, B0.  B0's reads come mostly from L2: DRAM traffic measured
-// 1.04x (FP32 storage) and 1.15x (FP64) the algorithmic 24 / 40 B/row at
-// 262144 x 512.
-// Every recurrence is the expression of k_tile.cuh; the two kernels agree to
-// rounding (bit for bit where the compiler contracts the same multiply-adds).
-// Needs NSEG = n_row / 16 even, 8 <= NSEG <= 32 (periodic: a power of two),
-// n_sys * elem a multiple of 16 bytes and 16-byte aligned arrays; SYS = 32, 64
-// or 128 for H in (8, 16], (4, 8] or [4, 4].
+// The ring is that of k_tile.cuh (full / empty mbarriers per stage, refills
+// issued by a rotating producer warp), with unhinted polls.  A, B, C, D are
+// read once.
+// Needs NSEG = n_row / 32 <= 16 (periodic: a power of two), n_sys * elem a
+// multiple of 16 bytes and 16-byte aligned arrays; SYS = 16 (NSEG = 16) to 256
+// systems, so that a CTA has 256 to 512 threads.
+//
+// Measured on B200 (262144 x 512): FP64 0.81 ms, FP32 storage 0.52 ms, 102 % and
+// 95 % of the copy bandwidth at the algorithmic 40 / 24 bytes a row (before,
+// with half the rows eliminated a second time from L2: 1.16 / 0.88 ms; the
+// DRAM moved 1.15x the bytes and each row's arithmetic ran 1.5 times).  Bound by
+// DRAM; with 6 / 5 / 4 ring stages of 32 KB it takes 0.811 / 0.815 / 0.857 ms.
 #pragma once
 
 #include "btdma_common.cuh"
@@ -38,14 +40,76 @@
 
 namespace btdma {
 
+constexpr int WIDE_M = 32;      // rows per sub-segment (per thread)
+constexpr int WIDE_TROWS = 20;  // rows whose state goes to tensor memory (the first ones)
+constexpr int WIDE_TCOLS = WIDE_TROWS * 6;  // columns of a warp: 3 doubles a row
+
 // Shared memory: ring (NST stages x 4 arrays x RPS x T elements) + reduced rows
 // (6 x NSEG x (SYS + 1) doubles; x_first / x_last reuse fields 0 and 1) +
-// 2 NST mbarriers.
+// 2 NST mbarriers + the tensor-memory address.
 __host__ __device__ __forceinline__ size_t tile_wide_smem_bytes(int sys, int nseg, int nst,
                                                                 int elem) {
-    const size_t t = (size_t)sys * (nseg / 2);
+    const size_t t = (size_t)sys * nseg;
     return (size_t)nst * 4 * tile_rps(elem) * t * elem + 6ull * nseg * (sys + 1) * sizeof(double) +
-           2ull * nst * sizeof(uint64_t) + 128;
+           2ull * nst * sizeof(uint64_t) + 16 + 128;
+}
+
+// ------------------------------------------------------------- tensor memory
+// Columns a CTA of `warps` warps allocates (a power of two >= 32).
+__host__ __device__ __forceinline__ int wide_tmem_cols(int warps) {
+    int c = 32;
+    while (c < (warps + 3) / 4 * WIDE_TCOLS) c <<= 1;
+    return c;
+}
+// One warp; the address of the columns is written to *dst (shared memory).  The
+// call waits while another CTA on the SM holds the columns.
+__device__ __forceinline__ void tmem_alloc(uint32_t* dst, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(dst)),
+                 "r"(cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() {
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// 4 doubles of every lane to / from 8 columns of the warp's lanes.  All lanes of
+// the warp call them together.
+__device__ __forceinline__ void tmem_store4(uint32_t addr, const double (&v)[4]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr),
+        "r"(__double2loint(v[0])), "r"(__double2hiint(v[0])), "r"(__double2loint(v[1])),
+        "r"(__double2hiint(v[1])), "r"(__double2loint(v[2])), "r"(__double2hiint(v[2])),
+        "r"(__double2loint(v[3])), "r"(__double2hiint(v[3]))
+        : "memory");
+}
+// The registers are valid after tmem_wait_ld on them.
+__device__ __forceinline__ void tmem_load4(uint32_t addr, uint32_t (&w)[8]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]),
+          "=r"(w[7])
+        : "r"(addr)
+        : "memory");
+}
+// Waits for the warp's loads; the registers pass through, so that no use of
+// them moves above it.
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&u)[8], uint32_t (&v)[8],
+                                             uint32_t (&w)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(u[0]), "+r"(u[1]), "+r"(u[2]), "+r"(u[3]), "+r"(u[4]), "+r"(u[5]),
+                   "+r"(u[6]), "+r"(u[7]), "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]),
+                   "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(w[0]), "+r"(w[1]),
+                   "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "+r"(w[6]), "+r"(w[7])
+                 :
+                 : "memory");
+}
+__device__ __forceinline__ double tmem_word(const uint32_t (&w)[8], int i) {
+    return __hiloint2double((int)w[2 * i + 1], (int)w[2 * i]);
 }
 
 // Running state of one sub-segment's forward pass (rows 0 .. M-1).
@@ -57,11 +121,9 @@ struct WideFwd {
 };
 
 // Row k of the forward pass (the expressions of k_tile.cuh's loop, FP64).
-// KEEP: store alpha, gamma, delta of the row in al / ga / de.
-template <bool KEEP>
 __device__ __forceinline__ void wide_row(WideFwd& f, int k, double a, double b, double cc,
-                                         double d, double* al, double* ga, double* de) {
-    constexpr int M = TILE_MT;
+                                         double d) {
+    constexpr int M = WIDE_M;
     if (k == 0) {
         const double ib = rcp_nr(b);
         f.ab0 = a * ib;
@@ -90,13 +152,6 @@ __device__ __forceinline__ void wide_row(WideFwd& f, int k, double a, double b, 
         f.gap = g;
         f.dep = e;
     }
-    if constexpr (KEEP) {
-        if (k >= 1) {
-            al[k] = f.alp;
-            ga[k] = f.gap;
-            de[k] = f.dep;
-        }
-    }
 }
 
 // The two reduced rows of a finished sub-segment into red[f][q][s].
@@ -111,21 +166,20 @@ __device__ __forceinline__ void wide_reduced(const WideFwd& f, double* w, int fs
     w[5 * fstride] = f.dep;
 }
 
-// FILT: Filtered's reduced system (as tile_f64_kernel's FILT).
+// FILT: Filtered's reduced system (as tile_f64_kernel's FILT; the mode's
+// segment length counts 32-row sub-segments here).
 template <int SYS, bool CYCLIC, typename TIN, bool FILT = false>
 __global__ void __launch_bounds__(TILE_MAX_THREADS, 1)
 tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmD,
                  const TileArgs args) {
-    constexpr int M = TILE_MT;
+    constexpr int M = WIDE_M, TR = WIDE_TROWS;
     constexpr int RPS = tile_rps((int)sizeof(TIN));
-    constexpr int SPG = M / RPS;    // stages per half sweep
-    constexpr int SPT = 3 * SPG;    // stages per group: A0, A1, B0
+    constexpr int SPG = M / RPS;  // stages per group
     constexpr int RP = SYS + 1;
     extern __shared__ unsigned char smem_raw[];
     const int nseg = args.nseg, nst = args.nst;
-    const int H = nseg / 2;
-    const int T = SYS * H;  // == blockDim.x
+    const int T = SYS * nseg;  // == blockDim.x, whole warps
     const int W = tile_lanes(nseg);
     const int fstride = nseg * RP;
 
@@ -135,13 +189,14 @@ tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     double* red = reinterpret_cast<double*>(ring + (size_t)nst * sstride);
     uint64_t* full = reinterpret_cast<uint64_t*>(red + 6 * fstride);
     uint64_t* empty = full + nst;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(empty + nst);
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
-    const int nwarps = (T + 31) / 32;
+    const int nwarps = T / 32;
     const int s = tid % SYS;
-    const int ql = tid / SYS;
+    const int q = tid / SYS;
     const size_t ns = (size_t)args.n_sys;
 
     if (tid == 0) {
@@ -151,7 +206,13 @@ tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
         fence_mbar_init();
     }
+    if (warp == 0) tmem_alloc(tslot, (uint32_t)wide_tmem_cols(nwarps));
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tbase = *static_cast<volatile uint32_t*>(tslot);
+    // this warp's lanes (its quarter) and columns
+    const uint32_t tcol = tbase + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * WIDE_TCOLS;
 
     // a closed gate leaves the CTA without groups (TILE_MODE_GATE_ZERO: the
     // gate is open while *gate == 0)
@@ -162,27 +223,25 @@ tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int n_my = (!gated_off && args.n_groups > (int)blockIdx.x)
                          ? (args.n_groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x
                          : 0;
-    const int total = n_my * SPT;
+    const int total = n_my * SPG;
     const uint32_t stage_bytes = (uint32_t)sstride * sizeof(TIN);
 
     auto issue = [&](int t) {  // one thread
         const int slot = t % nst;
-        const int g = (int)blockIdx.x + (t / SPT) * (int)gridDim.x;
-        const int u = t % SPT;
-        const int k0 = (u % SPG) * RPS;
-        const int z = (u / SPG) == 1 ? H : 0;
+        const int g = (int)blockIdx.x + (t / SPG) * (int)gridDim.x;
+        const int k0 = (t % SPG) * RPS;
         TIN* dst = ring + (size_t)slot * sstride;
         mbar_expect_tx(&full[slot], stage_bytes);
-        tma_load_3d(dst + 0 * RPS * T, &tmA, g * SYS, k0, z, &full[slot]);
-        tma_load_3d(dst + 1 * RPS * T, &tmB, g * SYS, k0, z, &full[slot]);
-        tma_load_3d(dst + 2 * RPS * T, &tmC, g * SYS, k0, z, &full[slot]);
-        tma_load_3d(dst + 3 * RPS * T, &tmD, g * SYS, k0, z, &full[slot]);
+        tma_load_3d(dst + 0 * RPS * T, &tmA, g * SYS, k0, 0, &full[slot]);
+        tma_load_3d(dst + 1 * RPS * T, &tmB, g * SYS, k0, 0, &full[slot]);
+        tma_load_3d(dst + 2 * RPS * T, &tmC, g * SYS, k0, 0, &full[slot]);
+        tma_load_3d(dst + 3 * RPS * T, &tmD, g * SYS, k0, 0, &full[slot]);
     };
     bool ok = true;
     if (tid == 0)
         for (int t = 0; t < nst && t < total; ++t) issue(t);
 
-    const int toff = ql * RPS * SYS + s;
+    const int toff = q * RPS * SYS + s;
     const TIN* st = ring + toff;
     int slot = 0;
     uint32_t phase = 0;
@@ -226,35 +285,39 @@ tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int g = (int)blockIdx.x + it * (int)gridDim.x;
         const int sys = g * SYS + s;
         const bool valid = sys < args.n_sys;
-        const int q0 = ql, q1 = H + ql;
 
-        // ------------------------------------------------ A0: scalars only
+        // ------------------------------------------------------ forward pass
+        double al[M - TR], ga[M - TR], de[M - TR];  // rows TR .. M - 1
         {
             WideFwd f = {};
+            double ta[4], tg[4], td[4];  // rows of the 4-row block going to tensor memory
 #pragma unroll
             for (int j = 0; j < SPG; ++j) {
                 double a2[RPS], b2[RPS], c2[RPS], d2[RPS];
                 fetch(a2, b2, c2, d2);
 #pragma unroll
-                for (int r = 0; r < RPS; ++r)
-                    wide_row<false>(f, j * RPS + r, a2[r], b2[r], c2[r], d2[r], nullptr, nullptr,
-                                    nullptr);
+                for (int r = 0; r < RPS; ++r) {
+                    const int k = j * RPS + r;
+                    wide_row(f, k, a2[r], b2[r], c2[r], d2[r]);
+                    if (k < TR) {
+                        ta[k % 4] = f.alp;
+                        tg[k % 4] = f.gap;
+                        td[k % 4] = f.dep;
+                    } else {
+                        al[k - TR] = f.alp;
+                        ga[k - TR] = f.gap;
+                        de[k - TR] = f.dep;
+                    }
+                }
+                const int kn = (j + 1) * RPS;
+                if (kn <= TR && kn % 4 == 0) {
+                    __syncwarp();
+                    tmem_store4(tcol + (kn - 4) * 6, ta);
+                    tmem_store4(tcol + (kn - 4) * 6 + 8, tg);
+                    tmem_store4(tcol + (kn - 4) * 6 + 16, td);
+                }
             }
-            wide_reduced(f, red + q0 * RP + s, fstride);
-        }
-        // ------------------------------------------------ A1: state kept
-        double al[M], ga[M], de[M];
-        {
-            WideFwd f = {};
-#pragma unroll
-            for (int j = 0; j < SPG; ++j) {
-                double a2[RPS], b2[RPS], c2[RPS], d2[RPS];
-                fetch(a2, b2, c2, d2);
-#pragma unroll
-                for (int r = 0; r < RPS; ++r)
-                    wide_row<true>(f, j * RPS + r, a2[r], b2[r], c2[r], d2[r], al, ga, de);
-            }
-            wide_reduced(f, red + q1 * RP + s, fstride);
+            wide_reduced(f, red + q * RP + s, fstride);
         }
         __syncthreads();
 
@@ -289,42 +352,51 @@ tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
         __syncthreads();
 
-        // ------------------------------------------------ B1, B0
-        auto back = [&](int q) {
-            const double x_first = red[q * RP + s];
-            const double x_last = red[fstride + q * RP + s];
-            if (!valid) return;
-            double* xp = args.X + (size_t)(q * M + M - 1) * ns + sys;
-            *xp = x_last;
-            double xn = x_last;
-#pragma unroll
-            for (int k = M - 2; k >= 1; --k) {
-                xp -= ns;
-                xn = de[k] - al[k] * x_first - ga[k] * xn;
-                nonfinite = fma(xn, 0.0, nonfinite);
-                *xp = xn;
+        // ------------------------------------------------ back substitution
+        const double x_first = red[q * RP + s];
+        const double x_last = red[fstride + q * RP + s];
+        double* xp = args.X + (size_t)(q * M + M - 1) * ns + sys;
+        double xn = x_last;
+        // systems past the batch are zero-filled (0 / 0 pivots): nothing of them
+        // is stored or counted
+        auto put = [&](double x) {
+            if (valid) {
+                *xp = x;
+                nonfinite = fma(x, 0.0, nonfinite);
             }
             xp -= ns;
-            *xp = x_first;
-            nonfinite = fma(x_first, 0.0, fma(x_last, 0.0, nonfinite));
         };
-        back(q1);
-        {
-            WideFwd f = {};
+        put(x_last);
 #pragma unroll
-            for (int j = 0; j < SPG; ++j) {
-                double a2[RPS], b2[RPS], c2[RPS], d2[RPS];
-                fetch(a2, b2, c2, d2);
+        for (int k = M - 2; k >= TR; --k) {
+            xn = de[k - TR] - al[k - TR] * x_first - ga[k - TR] * xn;
+            put(xn);
+        }
+        __syncwarp();
+        tmem_wait_st();
 #pragma unroll
-                for (int r = 0; r < RPS; ++r)
-                    wide_row<true>(f, j * RPS + r, a2[r], b2[r], c2[r], d2[r], al, ga, de);
+        for (int k0 = TR - 4; k0 >= 0; k0 -= 4) {
+            uint32_t wa[8], wg[8], wd[8];
+            tmem_load4(tcol + k0 * 6, wa);
+            tmem_load4(tcol + k0 * 6 + 8, wg);
+            tmem_load4(tcol + k0 * 6 + 16, wd);
+            tmem_wait_ld(wa, wg, wd);
+#pragma unroll
+            for (int r = 3; r >= 0; --r) {
+                if (k0 + r == 0) continue;  // row 0 is x_first
+                xn = tmem_word(wd, r) - tmem_word(wa, r) * x_first - tmem_word(wg, r) * xn;
+                put(xn);
             }
         }
-        back(q0);
+        put(x_first);
     }
     if (nonfinite != 0.0) raise_status(args.status, ST_NONFINITE);
     if (!ok && tid == 0)
         for (int i = 0; i < nst; ++i) mbar_wait_bounded(&full[i], 0, nullptr, 1u << 8);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0) tmem_dealloc(tbase, (uint32_t)wide_tmem_cols(nwarps));
 }
 
 }  // namespace btdma

@@ -416,10 +416,10 @@ int btdma_segments(btdma_t h, int* P);
 
 /* Kernel shape of the PaScaL solves that run the register-tiled kernel
  * (FP64 and FP32 storage with FP64 arithmetic).  NARROW: SYS systems per CTA
- * with every row's elimination state in registers.  WIDE: twice the systems
- * per CTA (wider HBM row pieces), half of each group's rows read a second time
- * from L2 instead of held.  AUTO: the library's measured choice per shape.
- * Both return the same bits.  No counterpart in the reference. */
+ * with every row's elimination state in registers.  WIDE (n_row a multiple of
+ * 32, 128 to 512): twice the systems per CTA (wider HBM row pieces), part of
+ * the state in tensor memory.  AUTO: the library's measured choice per shape.
+ * Both return the same solution to rounding.  No counterpart in the reference. */
 enum btdma_tile_shape {
     BTDMA_TILE_AUTO = 0,
     BTDMA_TILE_NARROW = 1,
