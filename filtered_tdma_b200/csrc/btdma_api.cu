@@ -86,8 +86,17 @@ int check_sizes(btdma_t h, int n_sys, int n_row) {
     return BTDMA_OK;
 }
 
+// Whether the segment kernels take the batch (shared memory, grid).
+bool seg_fits(btdma_t h, int n_sys, int n_row, bool cyclic) {
+    return seg_smem_bytes(seg_mcap(n_row, h->P), h->P, cyclic, true, seg_reg_rows(n_row, h->P)) <=
+               (size_t)max_smem_optin() &&
+           (n_sys + SEG_S - 1) / SEG_S <= 65535;
+}
+
+// n_plan: systems of the whole batch this call solves a part of (btdma_solve_host's
+// chunks run the kernels the whole batch would).
 int solve_impl(btdma_t h, const double* A, const double* B, const double* C, const double* D,
-               double* X, int n_sys, int n_row, bool cyclic, cudaStream_t st) {
+               double* X, int n_sys, int n_row, bool cyclic, cudaStream_t st, int n_plan) {
     int rc = check_sizes(h, n_sys, n_row);
     if (rc) return rc;
     if (!A || !B || !C || !D || !X) return fail(BTDMA_ERR_ARG, "null array");
@@ -140,10 +149,22 @@ int solve_impl(btdma_t h, const double* A, const double* B, const double* C, con
     }
 
     if (h->method == BTDMA_PASCAL && !(h->flags & BTDMA_FLAG_REFERENCE_ORDER)) {
+        // Shapes the narrow kernel does not take and that the segment kernels
+        // would: the wide solve's general form, but for small batches of short
+        // segments, whose shorter sweeps are faster there (B200, P = 4: 512 x 50
+        // 9.5 us against 10.2, 2048 x 50 9.8 / 10.3, 8192 x 50 10.8 / 10.4).
+        const bool general = seg_fits(h, n_sys, n_row, cyclic) &&
+                             !(n_sys % 2 == 0 && n_plan <= 4096 &&
+                               (n_row + h->P - 1) / h->P <= 16);
         rc = try_tile<double>(A, B, C, D, X, n_sys, n_row, cyclic, h->status, st, false,
-                              nullptr, h->tile_shape);
+                              nullptr, h->tile_shape, 0, false, general, n_plan);
         if (rc < 0) return rc;
         if (rc == 1) return BTDMA_OK;
+        if (general && cyclic && h->tile_shape == BTDMA_TILE_AUTO) {
+            rc = tile_any_solve(A, B, C, D, X, n_sys, n_row, h->status, st);
+            if (rc < 0) return rc;
+            if (rc == 1) return BTDMA_OK;
+        }
     }
 
     // Filtered v2 on the tiled kernels: the reference's P segments are groups
@@ -413,7 +434,7 @@ int btdma_solve_host(btdma_t h, const double* hA, const double* hB, const double
         CK(cudaStreamWaitEvent(p->s[1], p->in[b], 0));
         if (i >= 2) CK(cudaStreamWaitEvent(p->s[1], p->out[b], 0));
         if ((rc = solve_impl(h, d, d + be, d + 2 * be, d + 3 * be, d + 4 * be, c, n_row,
-                             cyclic != 0, p->s[1]))) {
+                             cyclic != 0, p->s[1], n_sys))) {
             // copies already queued still reference the host arrays: order the
             // caller's stream after them before reporting the error
             const std::string msg = g_err;
@@ -439,18 +460,18 @@ int btdma_solve_host(btdma_t h, const double* hA, const double* hB, const double
 
 int btdma_solve(btdma_t h, const double* A, const double* B, const double* C, double* D,
                 int n_sys, int n_row, cudaStream_t stream) {
-    return solve_impl(h, A, B, C, D, D, n_sys, n_row, false, stream);
+    return solve_impl(h, A, B, C, D, D, n_sys, n_row, false, stream, n_sys);
 }
 
 int btdma_solve_cyclic(btdma_t h, const double* A, const double* B, const double* C, double* D,
                        int n_sys, int n_row, cudaStream_t stream) {
-    return solve_impl(h, A, B, C, D, D, n_sys, n_row, true, stream);
+    return solve_impl(h, A, B, C, D, D, n_sys, n_row, true, stream, n_sys);
 }
 
 int btdma_solve_out(btdma_t h, const double* A, const double* B, const double* C,
                     const double* D, double* X, int n_sys, int n_row, int cyclic,
                     cudaStream_t stream) {
-    return solve_impl(h, A, B, C, D, X, n_sys, n_row, cyclic != 0, stream);
+    return solve_impl(h, A, B, C, D, X, n_sys, n_row, cyclic != 0, stream, n_sys);
 }
 
 int btdma_solve_f32(btdma_t h, const float* A, const float* B, const float* C, const float* D,

@@ -29,6 +29,19 @@ using namespace btdma;
 int tile_solve_batch(const void* A, const void* B, const void* C, const void* D, int elem,
                      double* X, int n_sys, int n_row, unsigned* status, cudaStream_t st);
 
+// The wide solve's general form (btdma_wide.cu): row counts up to 4096, odd n_sys
+// (FP64).  narrow: the narrow kernel takes the shape too; n_plan: the batch size
+// the choice between them is made for (btdma_solve_host's chunks follow the whole
+// batch).  Returns as tile_solve_batch.
+template <typename TIN>
+int tile_wide_gen(const TIN* A, const TIN* B, const TIN* C, const TIN* D, double* X, int n_sys,
+                  int n_row, bool cyclic, unsigned* status, cudaStream_t st, bool narrow,
+                  int n_plan);
+// Periodic FP64 systems whose row count is not 32 x a power of two
+// (btdma_any.cu).  Returns as tile_solve_batch.
+int tile_any_solve(const double* A, const double* B, const double* C, const double* D, double* X,
+                   int n_sys, int n_row, unsigned* status, cudaStream_t st);
+
 struct btdma_handle {
     int method, P, precision, flags;
     int tile_shape = 0;  // BTDMA_TILE_AUTO / NARROW / WIDE (uniform PaScaL batches)
@@ -433,6 +446,8 @@ inline TilePlan tile_wide_plan(int n_row, int n_sys, bool cyclic, int elem, bool
 template <int SYS, bool CYCLIC, typename TIN, bool FILT = false>
 int launch_tile_wide(const CUtensorMap* maps, const TileArgs& a, cudaStream_t st) {
     auto kern = tile_wide_kernel<SYS, CYCLIC, TIN, FILT>;
+    WideMaps wm;
+    std::copy(maps, maps + 4, wm.full);
     static bool attr_done = false;
     if (!attr_done) {
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -444,7 +459,7 @@ int launch_tile_wide(const CUtensorMap* maps, const TileArgs& a, cudaStream_t st
     int nb = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, threads, smem));
     const int grid = std::min(num_sms() * std::max(1, nb), a.n_groups);
-    kern<<<grid, threads, smem, st>>>(maps[0], maps[1], maps[2], maps[3], a);
+    kern<<<grid, threads, smem, st>>>(wm, a, WideGen{});
     CK(cudaGetLastError());
     return BTDMA_OK;
 }
@@ -475,19 +490,33 @@ inline bool tma_ok_elem(const void* p, int n_sys, int elem) {
 // TC: arithmetic of the local sweeps; accumulate: X += solution; gate: the
 // kernel does nothing while *gate == 0 (gate_zero: while *gate != 0); filt_r >
 // 0: Filtered's reduced system with segments of filt_r sub-segments.
-// shape: BTDMA_TILE_* (the wide-box kernel serves FP64-arithmetic solves that
-// do not accumulate).
+// shape: BTDMA_TILE_* (the wide kernel serves FP64-arithmetic solves that do not
+// accumulate; its general form serves AUTO's exact ungated ones, and with
+// `general` also shapes the narrow kernel does not take).  n_plan: the batch size
+// AUTO chooses for (0: n_sys).
 template <typename TIN, typename TC = double>
 int try_tile(const TIN* A, const TIN* B, const TIN* C, const TIN* D, double* X, int n_sys,
              int n_row, bool cyclic, unsigned* status, cudaStream_t st, bool accumulate = false,
              const unsigned* gate = nullptr, int shape = BTDMA_TILE_NARROW, int filt_r = 0,
-             bool gate_zero = false) {
+             bool gate_zero = false, bool general = false, int n_plan = 0) {
     const int elem = (int)sizeof(TIN);
+    if (n_plan <= 0) n_plan = n_sys;
+    const bool aligned = tma_ok_elem(A, n_sys, elem) && tma_ok_elem(B, n_sys, elem) &&
+                         tma_ok_elem(C, n_sys, elem) && tma_ok_elem(D, n_sys, elem);
     bool wide = false;
     TilePlan pl;
-    if (shape != BTDMA_TILE_NARROW && sizeof(TC) == 8 && !accumulate) {
-        pl = tile_wide_plan(n_row, n_sys, cyclic, elem, shape == BTDMA_TILE_WIDE);
+    if (shape != BTDMA_TILE_NARROW && sizeof(TC) == 8 && !accumulate && aligned) {
+        pl = tile_wide_plan(n_row, n_plan, cyclic, elem, shape == BTDMA_TILE_WIDE);
         wide = pl.sys != 0 && filt_r % 2 == 0;  // whole 32-row sub-segments
+    }
+    if (!wide && shape == BTDMA_TILE_AUTO && sizeof(TC) == 8 && !accumulate && !gate &&
+        filt_r == 0) {
+        const bool narrow = aligned && tile_plan(n_row, cyclic, elem).sys != 0;
+        if (narrow || general) {
+            const int rc = tile_wide_gen<TIN>(A, B, C, D, X, n_sys, n_row, cyclic, status, st,
+                                              narrow, n_plan);
+            if (rc != 0) return rc;
+        }
     }
     if (!wide) {
         pl = tile_plan(n_row, cyclic, elem);
@@ -496,10 +525,7 @@ int try_tile(const TIN* A, const TIN* B, const TIN* C, const TIN* D, double* X, 
         while (pl.sys > 16 && pl.cl == 1 && (n_sys + pl.sys - 1) / pl.sys < num_sms())
             pl.sys >>= 1;
     }
-    if (pl.sys == 0) return 0;
-    if (!(tma_ok_elem(A, n_sys, elem) && tma_ok_elem(B, n_sys, elem) &&
-          tma_ok_elem(C, n_sys, elem) && tma_ok_elem(D, n_sys, elem)))
-        return 0;
+    if (pl.sys == 0 || !aligned) return 0;
     const int nsc = pl.nseg / pl.cl;  // sub-segments per TMA box: the CTA's share
     const int mt = wide ? WIDE_M : TILE_MT;
     CUtensorMap maps[4];

@@ -178,6 +178,117 @@ __device__ __forceinline__ void reduced_solve_filtered(double l0, double u0, dou
     xl = da + lk * db + rk * dc;
 }
 
+// The reduced system of n consecutive sub-segments with their outer couplings as
+// parameters, over the lanes of reduced_solve_shfl: lane p's unknowns are
+//   xF(p) = f[0] + lam f[1] + rho f[2],  xL(p) = d[0] + lam d[1] + rho d[2]
+// with lam the last unknown left of them and rho the first one right of them
+// (reduced_solve_filtered's three right-hand sides, one segment of n lanes).
+__device__ __forceinline__ void reduced_condense(double l0, double u0, double r0, double l1,
+                                                 double u1, double r1, int p, int n, int W,
+                                                 bool act, double (&f)[3], double (&d)[3]) {
+    const unsigned FULL = 0xffffffffu;
+    const bool first = p == 0, last = p == n - 1;
+    const double l0s = first ? 0.0 : l0, u1s = last ? 0.0 : u1;  // couplings inside
+    const double b0 = first ? -l0 : 0.0, c1 = last ? -u1 : 0.0;
+    const int pn = (p + 1) & (W - 1);
+    // the next sub-segment's first row (its b0 is 0: it is not the first)
+    const double l0n = __shfl_sync(FULL, l0, pn, W), u0n = __shfl_sync(FULL, u0, pn, W);
+    const double r0n = __shfl_sync(FULL, r0, pn, W);
+    const double ib = rcp_nr(1.0 - l1 * u0 - u1s * l0n);
+    double al = -l1 * l0s * ib, cl = -u1s * u0n * ib;
+    double da = (r1 - l1 * r0 - u1s * r0n) * ib, db = -l1 * b0 * ib, dc = c1 * ib;
+    if (!act) al = cl = da = db = dc = 0.0;
+    for (int dl = 1; dl < n; dl <<= 1) {
+        const bool vm = p - dl >= 0, vp = p + dl < n;
+        const int im = (p - dl) & (W - 1), ip = (p + dl) & (W - 1);
+        double lm = __shfl_sync(FULL, al, im, W), um = __shfl_sync(FULL, cl, im, W);
+        double lp = __shfl_sync(FULL, al, ip, W), up = __shfl_sync(FULL, cl, ip, W);
+        double am = __shfl_sync(FULL, da, im, W), ap = __shfl_sync(FULL, da, ip, W);
+        double bm = __shfl_sync(FULL, db, im, W), bp = __shfl_sync(FULL, db, ip, W);
+        double cm = __shfl_sync(FULL, dc, im, W), cp = __shfl_sync(FULL, dc, ip, W);
+        if (!vm) lm = um = am = bm = cm = 0.0;
+        if (!vp) lp = up = ap = bp = cp = 0.0;
+        const double ibl = rcp_nr(1.0 - al * um - cl * lp);
+        da = (da - al * am - cl * ap) * ibl;
+        db = (db - al * bm - cl * bp) * ibl;
+        dc = (dc - al * cm - cl * cp) * ibl;
+        const double nl = -al * lm * ibl;
+        cl = -cl * up * ibl;
+        al = nl;
+    }
+    const int pm = (p - 1) & (W - 1);
+    double xam = __shfl_sync(FULL, da, pm, W), xbm = __shfl_sync(FULL, db, pm, W);
+    double xcm = __shfl_sync(FULL, dc, pm, W);
+    if (first) xam = xbm = xcm = 0.0;
+    f[0] = r0 - l0s * xam - u0 * da;
+    f[1] = b0 - l0s * xbm - u0 * db;
+    f[2] = -l0s * xcm - u0 * dc;
+    d[0] = da;
+    d[1] = db;
+    d[2] = dc;
+}
+
+// The outer unknowns of n condensed blocks of one system, lane r of a group of W
+// holding block r's first and last rows
+//   F_r = f[0] + L_{r-1} f[1] + F_{r+1} f[2],  L_r = d[0] + L_{r-1} d[1] + F_{r+1} d[2]:
+// lam = L_{r-1} and rho = F_{r+1} (0 outside the system unless CYCLIC).  Block by
+// block, L_r = p + pl L_{-1} + s F_{r+1} and F_r = P + Pl L_{-1} + S F_{r+1};
+// periodic systems close the chain with a 2 x 2 system in L_{-1} = L_{n-1} and
+// F_n = F_0.  Every lane of the warp calls it.
+template <bool CYCLIC>
+__device__ __forceinline__ void reduced_outer(const double (&f)[3], const double (&d)[3], int r,
+                                              int n, int W, double& lam, double& rho) {
+    const unsigned FULL = 0xffffffffu;
+    double P = f[0], S = f[2], p = d[0], s = d[2];
+    double Pl = CYCLIC ? f[1] : 0.0, pl = CYCLIC ? d[1] : 0.0;  // of block 0
+    for (int k = 1; k < n; ++k) {
+        const double pm = __shfl_sync(FULL, p, k - 1, W), sm = __shfl_sync(FULL, s, k - 1, W);
+        const double plm = CYCLIC ? __shfl_sync(FULL, pl, k - 1, W) : 0.0;
+        if (r == k) {
+            const double ib = rcp_nr(1.0 - f[1] * sm);
+            P = (f[0] + f[1] * pm) * ib;
+            S = f[2] * ib;
+            p = d[0] + d[1] * (pm + sm * P);
+            s = d[1] * sm * S + d[2];
+            if constexpr (CYCLIC) {
+                Pl = f[1] * plm * ib;
+                pl = d[1] * (plm + sm * Pl);
+            }
+        }
+    }
+    double x = P, y = Pl, z = S;  // F_r = x + y L_{-1} + z F_n
+    for (int k = n - 2; k >= 0; --k) {
+        const double xn = __shfl_sync(FULL, x, k + 1, W);
+        const double yn = CYCLIC ? __shfl_sync(FULL, y, k + 1, W) : 0.0;
+        const double zn = CYCLIC ? __shfl_sync(FULL, z, k + 1, W) : 0.0;
+        if (r == k) {
+            x = P + S * xn;
+            if constexpr (CYCLIC) {
+                y = Pl + S * yn;
+                z = S * zn;
+            }
+        }
+    }
+    double fr = x;
+    double L0 = 0.0, Fn = 0.0;  // L_{-1}, F_n
+    if constexpr (CYCLIC) {
+        const double x0 = __shfl_sync(FULL, x, 0, W), y0 = __shfl_sync(FULL, y, 0, W);
+        const double z0 = __shfl_sync(FULL, z, 0, W);
+        const double pe = __shfl_sync(FULL, p, n - 1, W), ple = __shfl_sync(FULL, pl, n - 1, W);
+        const double se = __shfl_sync(FULL, s, n - 1, W);
+        const double id = rcp_nr((1.0 - z0) * (1.0 - ple) - y0 * se);
+        Fn = (x0 * (1.0 - ple) + y0 * pe) * id;
+        L0 = ((1.0 - z0) * pe + se * x0) * id;
+        fr = x + y * L0 + z * Fn;
+    }
+    const int rm = (r - 1) & (W - 1), rp = (r + 1) & (W - 1);
+    const double pm = __shfl_sync(FULL, p, rm, W), sm = __shfl_sync(FULL, s, rm, W);
+    const double plm = CYCLIC ? __shfl_sync(FULL, pl, rm, W) : 0.0;
+    const double fn = __shfl_sync(FULL, fr, rp, W);
+    lam = r == 0 ? L0 : pm + plm * L0 + sm * fr;
+    rho = r == n - 1 ? Fn : fn;
+}
+
 // The matrix steps of reduced_solve_shfl for one lane, written to lt[0 .. 5 +
 // 3 * levels) (the lane table of a matrix shared by every system, see
 // reduced_solve_rhs).  Every lane of the warp calls it with the same nseg

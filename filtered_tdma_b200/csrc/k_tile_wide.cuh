@@ -34,6 +34,10 @@
 // DRAM; with 6 / 5 / 4 ring stages of 32 KB it takes 0.811 / 0.815 / 0.857 ms.
 #pragma once
 
+#include <cooperative_groups.h>
+
+#include <type_traits>
+
 #include "btdma_common.cuh"
 #include "k_reduced.cuh"
 #include "k_tile.cuh"
@@ -44,14 +48,56 @@ constexpr int WIDE_M = 32;      // rows per sub-segment (per thread)
 constexpr int WIDE_TROWS = 20;  // rows whose state goes to tensor memory (the first ones)
 constexpr int WIDE_TCOLS = WIDE_TROWS * 6;  // columns of a warp: 3 doubles a row
 
-// Shared memory: ring (NST stages x 4 arrays x RPS x T elements) + reduced rows
-// (6 x NSEG x (SYS + 1) doubles; x_first / x_last reuse fields 0 and 1) +
-// 2 NST mbarriers + the tensor-memory address.
+// The general form (GEN) takes any n_row and odd n_sys, and with CLUSTER systems
+// longer than a CTA holds:
+//   tail      the sub-segment with the system's last rows arrives by boxes of its
+//             own (rows past the end are zero-filled; there B becomes 1, which
+//             leaves identity rows, x = 0).  C's boxes end one row earlier, so the
+//             unused coupling of the last row is 0 whatever the array holds.
+//   odd       with an odd n_sys every other row is 8 bytes off TMA's 16: rows are
+//             taken in pairs, as a row of 2 n_sys elements whose stride suits
+//             TMA, the odd row from x = n_sys + first system - 1 (even), in boxes
+//             two elements wider.
+//   cluster   CL CTAs each own NSC consecutive sub-segments of the same systems.
+//             A CTA solves its own reduced system with its two outer couplings as
+//             parameters (reduced_condense): its first and last unknown become
+//             linear in the left neighbour's last and the right neighbour's first
+//             unknown.  These six numbers a system are published in shared memory
+//             (double buffered); every CTA signals its peers' mbarriers once a
+//             group, reads all CL of them and eliminates over the CTAs in lane
+//             registers (reduced_outer).
+struct WideMaps {
+    CUtensorMap full[4];  // A, B, C, D: boxes of the CTA's sub-segments
+};
+struct WideMapsGen {
+    CUtensorMap full[4];
+    CUtensorMap less[4];  // the last CTA: its sub-segments before the tail one
+    CUtensorMap tail[4];  // the tail one (and all-identity ones after it)
+    CUtensorMap last[4];  // odd n_sys: the tail's unpaired last row
+};
+struct WideGen {
+    int tail;   // rows of the tail sub-segment (0: periodic, none)
+    int nl;     // sub-segments before it in the last CTA
+    int empty;  // bit f: array f has no (pair of) rows in the tail's box
+};
+
+// Elements of a ring stage; odd n_sys: a box per array and row of NSC pieces of
+// SYS + 2, the tail's box on a 128-byte boundary of its own.
+__host__ __device__ __forceinline__ int wide_odd_box(int sys, int nseg) {
+    return (nseg * (sys + 2) + 15) / 16 * 16 + 16;
+}
+__host__ __device__ __forceinline__ int wide_stage_elems(int sys, int nseg, int elem, bool odd) {
+    return odd ? 8 * wide_odd_box(sys, nseg) : 4 * tile_rps(elem) * sys * nseg;
+}
+// Shared memory: ring + reduced rows (6 x NSEG x (SYS + 1) doubles; x_first /
+// x_last reuse fields 0 and 1) + published rows [2][6][SYS] and outer unknowns
+// [2][SYS] (clusters) + mbarriers + the tensor-memory address.
 __host__ __device__ __forceinline__ size_t tile_wide_smem_bytes(int sys, int nseg, int nst,
-                                                                int elem) {
-    const size_t t = (size_t)sys * nseg;
-    return (size_t)nst * 4 * tile_rps(elem) * t * elem + 6ull * nseg * (sys + 1) * sizeof(double) +
-           2ull * nst * sizeof(uint64_t) + 16 + 128;
+                                                                int elem, bool odd = false,
+                                                                int cl = 1) {
+    return (size_t)nst * wide_stage_elems(sys, nseg, elem, odd) * elem +
+           6ull * nseg * (sys + 1) * sizeof(double) + (cl > 1 ? 14ull * sys * sizeof(double) : 0) +
+           (2ull * nst + 2) * sizeof(uint64_t) + 16 + 128;
 }
 
 // ------------------------------------------------------------- tensor memory
@@ -112,6 +158,39 @@ __device__ __forceinline__ double tmem_word(const uint32_t (&w)[8], int i) {
     return __hiloint2double((int)w[2 * i + 1], (int)w[2 * i]);
 }
 
+// One arrival on the mbarrier at the same shared-memory offset in CTA `rank` of
+// the cluster, releasing this thread's (and, after a block barrier, the CTA's)
+// earlier writes to the cluster.
+__device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, int rank) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(bar)),
+                 "r"(rank));
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote)
+                 : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+static __device__ __noinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity,
+                                                      unsigned* status) {
+    for (uint32_t it = 0; it < (1u << 22); ++it) {
+        if (mbar_try_wait_cluster(bar, parity)) return true;
+        if (status && (it & 1023u) == 1023u &&
+            (*reinterpret_cast<volatile unsigned*>(status) & ST_TIMEOUT))
+            return false;
+    }
+    raise_status(status, ST_TIMEOUT);
+    return false;
+}
+
 // Running state of one sub-segment's forward pass (rows 0 .. M-1).
 struct WideFwd {
     double ab0, cb0, db0;  // row 0 scaled by its pivot
@@ -166,30 +245,40 @@ __device__ __forceinline__ void wide_reduced(const WideFwd& f, double* w, int fs
     w[5 * fstride] = f.dep;
 }
 
-// FILT: Filtered's reduced system (as tile_f64_kernel's FILT; the mode's
-// segment length counts 32-row sub-segments here).
-template <int SYS, bool CYCLIC, typename TIN, bool FILT = false>
+// FILT: Filtered's reduced system (as tile_f64_kernel's FILT; the mode's segment
+// length counts 32-row sub-segments here).
+template <int SYS, bool CYCLIC, typename TIN, bool FILT = false, bool GEN = false,
+          bool CLUSTER = false>
 __global__ void __launch_bounds__(TILE_MAX_THREADS, 1)
-tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmD,
-                 const TileArgs args) {
+tile_wide_kernel(const __grid_constant__ std::conditional_t<GEN, WideMapsGen, WideMaps> maps,
+                 const TileArgs args, const WideGen gen) {
+    namespace cg = cooperative_groups;
+    static_assert(!FILT || !GEN, "Filtered segments are whole sub-segments");
+    static_assert(!CLUSTER || GEN, "clusters run the general form");
     constexpr int M = WIDE_M, TR = WIDE_TROWS;
     constexpr int RPS = tile_rps((int)sizeof(TIN));
     constexpr int SPG = M / RPS;  // stages per group
     constexpr int RP = SYS + 1;
+    constexpr bool PAD = GEN && !CYCLIC;
     extern __shared__ unsigned char smem_raw[];
-    const int nseg = args.nseg, nst = args.nst;
+    const int nseg = args.nseg, nst = args.nst;  // nseg: sub-segments of this CTA
+    const int cl = CLUSTER ? args.cl : 1;
     const int T = SYS * nseg;  // == blockDim.x, whole warps
     const int W = tile_lanes(nseg);
     const int fstride = nseg * RP;
+    const bool odd = GEN && sizeof(TIN) == 8 && (args.n_sys & 1) != 0;
+    const int bx = odd ? wide_odd_box(SYS, nseg) : 0;
 
     TIN* ring = reinterpret_cast<TIN*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-    const int sstride = 4 * RPS * T;  // elements per stage
+    const int sstride = odd ? 8 * bx : 4 * RPS * T;  // elements per stage
     double* red = reinterpret_cast<double*>(ring + (size_t)nst * sstride);
-    uint64_t* full = reinterpret_cast<uint64_t*>(red + 6 * fstride);
+    double* pub = red + 6 * fstride;                 // [2][6][SYS]
+    double* outer = pub + (CLUSTER ? 12 * SYS : 0);  // [2][SYS]
+    uint64_t* full = reinterpret_cast<uint64_t*>(outer + (CLUSTER ? 2 * SYS : 0));
     uint64_t* empty = full + nst;
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(empty + nst);
+    uint64_t* xbar = empty + nst;  // [2]: the peers' published rows of a group
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(xbar + 2);
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -198,21 +287,32 @@ tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int s = tid % SYS;
     const int q = tid / SYS;
     const size_t ns = (size_t)args.n_sys;
+    const int c = CLUSTER ? (int)cg::this_cluster().block_rank() : 0;
+    const int cid = CLUSTER ? (int)blockIdx.x / cl : (int)blockIdx.x;
+    const int ncid = CLUSTER ? (int)gridDim.x / cl : (int)gridDim.x;
+    const int r0 = (c * nseg + q) * M;  // first row of the sub-segment
+    // PAD: rows of the sub-segment that the system has (<= 0: none)
+    const int mlen = PAD ? args.n_row - r0 : M;
+    const bool tailed = PAD && c == cl - 1;
+    const int nmain = tailed ? gen.nl : nseg;  // sub-segments of the main boxes
 
     if (tid == 0) {
         for (int i = 0; i < nst; ++i) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], nwarps);
         }
+        mbar_init(&xbar[0], cl);
+        mbar_init(&xbar[1], cl);
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(tslot, (uint32_t)wide_tmem_cols(nwarps));
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tbase = *static_cast<volatile uint32_t*>(tslot);
+    if constexpr (CLUSTER) tile_cluster_sync(cl);  // the peers' mbarriers are ready
     // this warp's lanes (its quarter) and columns
-    const uint32_t tcol = tbase + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * WIDE_TCOLS;
+    const uint32_t tcol = *static_cast<volatile uint32_t*>(tslot) + ((uint32_t)(warp & 3) << 21) +
+                          (uint32_t)(warp >> 2) * WIDE_TCOLS;
 
     // a closed gate leaves the CTA without groups (TILE_MODE_GATE_ZERO: the
     // gate is open while *gate == 0)
@@ -220,28 +320,61 @@ tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                            ((*static_cast<const volatile unsigned*>(args.gate) == 0u) !=
                             ((args.mode & TILE_MODE_GATE_ZERO) != 0));
     const int filt_r = FILT ? (args.mode >> TILE_MODE_FILT_SHIFT) & 255 : 0;  // lanes a segment
-    const int n_my = (!gated_off && args.n_groups > (int)blockIdx.x)
-                         ? (args.n_groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x
+    const int n_my = (!gated_off && args.n_groups > cid)
+                         ? (args.n_groups - cid + ncid - 1) / ncid
                          : 0;
     const int total = n_my * SPG;
-    const uint32_t stage_bytes = (uint32_t)sstride * sizeof(TIN);
+    const uint32_t stage_bytes =
+        odd ? 8u * nseg * (SYS + 2) * sizeof(TIN) : (uint32_t)sstride * sizeof(TIN);
 
-    auto issue = [&](int t) {  // one thread
+    // Stage t: one thread, or (GEN) a warp: lane = array + 4 (tail) + 8 (odd row).
+    auto issue = [&](int t) {
         const int slot = t % nst;
-        const int g = (int)blockIdx.x + (t / SPG) * (int)gridDim.x;
+        const int g0 = (cid + (t / SPG) * ncid) * SYS;
         const int k0 = (t % SPG) * RPS;
         TIN* dst = ring + (size_t)slot * sstride;
-        mbar_expect_tx(&full[slot], stage_bytes);
-        tma_load_3d(dst + 0 * RPS * T, &tmA, g * SYS, k0, 0, &full[slot]);
-        tma_load_3d(dst + 1 * RPS * T, &tmB, g * SYS, k0, 0, &full[slot]);
-        tma_load_3d(dst + 2 * RPS * T, &tmC, g * SYS, k0, 0, &full[slot]);
-        tma_load_3d(dst + 3 * RPS * T, &tmD, g * SYS, k0, 0, &full[slot]);
+        if constexpr (GEN) {
+            if (lane == 0) mbar_expect_tx(&full[slot], stage_bytes);
+            __syncwarp();
+            const int f = lane & 3, tl = (lane >> 2) & 1, par = lane >> 3;
+            if (par > (odd ? 1 : 0) || (tl ? !tailed : nmain == 0)) return;
+            const CUtensorMap* mp = tl ? &maps.tail[f] : (tailed ? &maps.less[f] : &maps.full[f]);
+            int x = g0, y = odd ? k0 >> 1 : k0, z = tl ? 0 : c * nseg;
+            if (odd) {
+                dst += (f * 2 + par) * bx + (tl ? (nmain * (SYS + 2) + 15) / 16 * 16 : 0);
+                if (par) x += args.n_sys - 1;
+            } else {
+                dst += f * RPS * T + (tl ? nmain * RPS * SYS : 0);
+            }
+            if (tl) {
+                const int rows = gen.tail - (f == 2 ? 1 : 0);  // C: not its last row
+                if (odd && !par && (rows & 1) && y == rows >> 1) {
+                    mp = &maps.last[f];
+                    y = 0;
+                } else {
+                    y += (gen.empty >> f) & 1;  // nothing there: past the map's one row
+                }
+            }
+            tma_load_3d(dst, mp, x, y, z, &full[slot]);
+        } else {
+            mbar_expect_tx(&full[slot], stage_bytes);
+            tma_load_3d(dst + 0 * RPS * T, &maps.full[0], g0, k0, 0, &full[slot]);
+            tma_load_3d(dst + 1 * RPS * T, &maps.full[1], g0, k0, 0, &full[slot]);
+            tma_load_3d(dst + 2 * RPS * T, &maps.full[2], g0, k0, 0, &full[slot]);
+            tma_load_3d(dst + 3 * RPS * T, &maps.full[3], g0, k0, 0, &full[slot]);
+        }
     };
     bool ok = true;
-    if (tid == 0)
+    if (GEN ? warp == 0 : tid == 0)
         for (int t = 0; t < nst && t < total; ++t) issue(t);
 
-    const int toff = q * RPS * SYS + s;
+    // this thread's rows of a stage: array f, row r at st + f * fstep + r * rstep
+    const int toff = odd ? (q < nmain ? q * (SYS + 2)
+                                      : (nmain * (SYS + 2) + 15) / 16 * 16 +
+                                            (q - nmain) * (SYS + 2)) + s
+                         : q * RPS * SYS + s;
+    const int rstep = odd ? bx + 1 : SYS;
+    const int fstep = odd ? 2 * bx : RPS * T;
     const TIN* st = ring + toff;
     int slot = 0;
     uint32_t phase = 0;
@@ -255,13 +388,20 @@ tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (ok) ok = mbar_wait_bounded_spin(&full[slot], phase, args.status);
 #pragma unroll
         for (int r = 0; r < RPS; ++r) {
-            a2[r] = (double)st[0 * RPS * T + r * SYS];
-            b2[r] = (double)st[1 * RPS * T + r * SYS];
-            c2[r] = (double)st[2 * RPS * T + r * SYS];
-            d2[r] = (double)st[3 * RPS * T + r * SYS];
+            a2[r] = (double)st[0 * fstep + r * rstep];
+            b2[r] = (double)st[1 * fstep + r * rstep];
+            c2[r] = (double)st[2 * fstep + r * rstep];
+            d2[r] = (double)st[3 * fstep + r * rstep];
         }
         __syncwarp();
-        if (lane == 0) {
+        if constexpr (GEN) {
+            if (lane == 0) mbar_arrive(&empty[slot]);
+            if (warp == tw && t >= 1 && t - 1 + nst < total) {
+                if (ok) ok = mbar_wait_bounded_spin(&empty[pslot], pphase, args.status);
+                if (ok) issue(t - 1 + nst);
+                __syncwarp();
+            }
+        } else if (lane == 0) {
             mbar_arrive(&empty[slot]);
             if (t >= 1 && warp == tw && t - 1 + nst < total && ok) {
                 ok = mbar_wait_bounded_spin(&empty[pslot], pphase, args.status);
@@ -282,7 +422,7 @@ tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
     double nonfinite = 0.0;
     for (int it = 0; it < n_my; ++it) {
-        const int g = (int)blockIdx.x + it * (int)gridDim.x;
+        const int g = cid + it * ncid;
         const int sys = g * SYS + s;
         const bool valid = sys < args.n_sys;
 
@@ -298,6 +438,7 @@ tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
                 for (int r = 0; r < RPS; ++r) {
                     const int k = j * RPS + r;
+                    if constexpr (PAD) b2[r] = k < mlen ? b2[r] : 1.0;
                     wide_row(f, k, a2[r], b2[r], c2[r], d2[r]);
                     if (k < TR) {
                         ta[k % 4] = f.alp;
@@ -317,6 +458,7 @@ tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     tmem_store4(tcol + (kn - 4) * 6 + 16, td);
                 }
             }
+            if constexpr (PAD) f.ab0 = r0 == 0 ? 0.0 : f.ab0;  // no row above the first
             wide_reduced(f, red + q * RP + s, fstride);
         }
         __syncthreads();
@@ -325,52 +467,104 @@ tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         {
             const int per_pass = T / W;  // systems per pass
             const int p = tid % W;
+            double* pb = pub + (it & 1) * 6 * SYS;
             for (int base = 0; base < SYS; base += per_pass) {
                 const int sp = base + tid / W;
                 const bool act = sp < SYS && p < nseg;
-                double l0 = 0, u0 = 0, r0 = 0, l1 = 0, u1 = 0, r1 = 0;
+                double l0 = 0, u0 = 0, b0 = 0, l1 = 0, u1 = 0, b1 = 0;
                 double* src = red + p * RP + sp;
                 if (act) {
                     l0 = src[0 * fstride];
                     u0 = src[1 * fstride];
-                    r0 = src[2 * fstride];
+                    b0 = src[2 * fstride];
                     l1 = src[3 * fstride];
                     u1 = src[4 * fstride];
-                    r1 = src[5 * fstride];
+                    b1 = src[5 * fstride];
                 }
-                double xf, xl;
-                if constexpr (FILT)
-                    reduced_solve_filtered<CYCLIC>(l0, u0, r0, l1, u1, r1, p, nseg, W, filt_r,
-                                                   act, xf, xl);
-                else
-                    reduced_solve_shfl<CYCLIC>(l0, u0, r0, l1, u1, r1, p, nseg, W, act, xf, xl);
-                if (act) {  // over the fields this thread has read
-                    src[0] = xf;
-                    src[fstride] = xl;
+                if constexpr (CLUSTER) {
+                    double f[3], d[3];
+                    reduced_condense(l0, u0, b0, l1, u1, b1, p, nseg, W, act, f, d);
+                    if (act) {  // over the fields this thread has read
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) {
+                            src[i * fstride] = f[i];
+                            src[(3 + i) * fstride] = d[i];
+                            if (p == 0) pb[i * SYS + sp] = f[i];
+                            if (p == nseg - 1) pb[(3 + i) * SYS + sp] = d[i];
+                        }
+                    }
+                } else {
+                    double xf, xl;
+                    if constexpr (FILT)
+                        reduced_solve_filtered<CYCLIC>(l0, u0, b0, l1, u1, b1, p, nseg, W, filt_r,
+                                                       act, xf, xl);
+                    else
+                        reduced_solve_shfl<CYCLIC>(l0, u0, b0, l1, u1, b1, p, nseg, W, act, xf,
+                                                   xl);
+                    if (act) {
+                        src[0] = xf;
+                        src[fstride] = xl;
+                    }
+                }
+            }
+            if constexpr (CLUSTER) {
+                __syncthreads();  // the CTA's rows are published
+                if (tid < cl) mbar_arrive_cluster(&xbar[it & 1], tid);
+                if (ok) ok = mbar_wait_cluster(&xbar[it & 1], (it >> 1) & 1, args.status);
+                // the outer unknowns of every CTA of a system, one lane a CTA
+                const int WC = tile_lanes(cl);
+                const int r = tid % WC;
+                for (int base = 0; base < SYS; base += T / WC) {
+                    const int sp = base + tid / WC;
+                    double f[3] = {0, 0, 0}, d[3] = {0, 0, 0};
+                    if (sp < SYS && r < cl) {
+                        const double* src = cg::this_cluster().map_shared_rank(pb, r) + sp;
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) {
+                            f[i] = src[i * SYS];
+                            d[i] = src[(3 + i) * SYS];
+                        }
+                    }
+                    double lam, rho;
+                    reduced_outer<CYCLIC>(f, d, r, cl, WC, lam, rho);
+                    if (sp < SYS && r == c) {
+                        outer[sp] = lam;
+                        outer[SYS + sp] = rho;
+                    }
                 }
             }
         }
         __syncthreads();
 
         // ------------------------------------------------ back substitution
-        const double x_first = red[q * RP + s];
-        const double x_last = red[fstride + q * RP + s];
-        double* xp = args.X + (size_t)(q * M + M - 1) * ns + sys;
+        double x_first, x_last;
+        {
+            const double* src = red + q * RP + s;
+            if constexpr (CLUSTER) {
+                const double lam = outer[s], rho = outer[SYS + s];
+                x_first = src[0] + lam * src[1 * fstride] + rho * src[2 * fstride];
+                x_last = src[3 * fstride] + lam * src[4 * fstride] + rho * src[5 * fstride];
+            } else {
+                x_first = src[0];
+                x_last = src[fstride];
+            }
+        }
+        double* xp = args.X + (size_t)(r0 + M - 1) * ns + sys;
         double xn = x_last;
         // systems past the batch are zero-filled (0 / 0 pivots): nothing of them
         // is stored or counted
-        auto put = [&](double x) {
-            if (valid) {
+        auto put = [&](int k, double x) {
+            if (valid && (!PAD || k < mlen)) {
                 *xp = x;
                 nonfinite = fma(x, 0.0, nonfinite);
             }
             xp -= ns;
         };
-        put(x_last);
+        put(M - 1, x_last);
 #pragma unroll
         for (int k = M - 2; k >= TR; --k) {
             xn = de[k - TR] - al[k - TR] * x_first - ga[k - TR] * xn;
-            put(xn);
+            put(k, xn);
         }
         __syncwarp();
         tmem_wait_st();
@@ -385,18 +579,20 @@ tile_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             for (int r = 3; r >= 0; --r) {
                 if (k0 + r == 0) continue;  // row 0 is x_first
                 xn = tmem_word(wd, r) - tmem_word(wa, r) * x_first - tmem_word(wg, r) * xn;
-                put(xn);
+                put(k0 + r, xn);
             }
         }
-        put(x_first);
+        put(0, x_first);
     }
     if (nonfinite != 0.0) raise_status(args.status, ST_NONFINITE);
-    if (!ok && tid == 0)
+    if (!ok && (GEN ? warp == 0 : tid == 0))
         for (int i = 0; i < nst; ++i) mbar_wait_bounded(&full[i], 0, nullptr, 1u << 8);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (warp == 0) tmem_dealloc(tbase, (uint32_t)wide_tmem_cols(nwarps));
+    if (warp == 0)
+        tmem_dealloc(*static_cast<volatile uint32_t*>(tslot), (uint32_t)wide_tmem_cols(nwarps));
+    if constexpr (CLUSTER) tile_cluster_sync(cl);  // peers may still read this CTA's rows
 }
 
 }  // namespace btdma
