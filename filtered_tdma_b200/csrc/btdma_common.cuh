@@ -154,6 +154,20 @@ static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parit
     return false;
 }
 
+// Before a ring stage is given back for its next TMA copy, the values read from it
+// must be in registers: a shared-memory load can wait behind a backlog of global
+// stores while the mbarrier arrival, which takes another path, overtakes it, and the
+// refill then lands under the load (seen on B200 as rare wrong groups right after a
+// back substitution's stores, with the release placed straight after the loads).
+// bits: the XOR of a word of every value loaded; zero: a 0 the compiler cannot see.
+// Returns 0, known only once every lane's loads have completed; the arrival's address
+// takes it in.
+__device__ __forceinline__ unsigned loads_done(unsigned bits, unsigned zero) {
+    return __any_sync(0xffffffffu, (bits & zero) != 0u) ? 1u : 0u;
+}
+__device__ __forceinline__ unsigned word_of(double v) { return (unsigned)__double2hiint(v); }
+__device__ __forceinline__ unsigned word_of(float v) { return (unsigned)__float_as_int(v); }
+
 // ------------------------------------------------------------------------ TMA
 // 2-D tiled load global -> this CTA's shared memory, completion on `bar`.
 // x = innermost coordinate (system index, a multiple of the tile width, so its

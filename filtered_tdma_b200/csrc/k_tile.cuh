@@ -340,6 +340,7 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const int n_clusters = (int)gridDim.x / cl;
     const int s = tid % SYS;  // forward / back-substitution mapping
     const int ql = tid / SYS;
+    const unsigned zero = (unsigned)args.n_sys >> 31;  // see loads_done
     // row stride of x: n_sys, or xrs through the layout map of the generated modes
     const size_t ns = (CONSTC && args.xblk > 0) ? (size_t)args.xrs : (size_t)args.n_sys;
 
@@ -574,6 +575,7 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             for (int j = 0; j < SPG; ++j) {
                 if (ok) ok = mbar_wait_bounded(&full[slot], phase, args.status);
                 TIN a2[RPS], b2[RPS], c2[RPS], d2[PR][RPS];  // widened where used
+                unsigned bits = 0;
 #pragma unroll
                 for (int r = 0; r < RPS; ++r) {
                     if constexpr (!CONSTC) {
@@ -588,11 +590,13 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                                             ((ql + h * hsc) * RPS + r) * TILE_HEAT_BOX_I + s + 1];
                         else
                             d2[h][r] = st[(NA - 1) * RPS * TS + h * hsc * RPS * SYS + r * SYS];
+                        bits ^= word_of(d2[h][r]);
                     }
+                    if constexpr (!CONSTC) bits ^= word_of(a2[r]) ^ word_of(b2[r]) ^ word_of(c2[r]);
                 }
-                __syncwarp();
+                const unsigned z = loads_done(bits, zero);
                 if (lane == 0) {
-                    mbar_arrive(&empty[slot]);
+                    mbar_arrive(&empty[slot] + z);
                     // Rotating producer: one stage later, warp (t % nwarps) refills
                     // the slot of stage t - 1 with stage t - 1 + nst once every warp
                     // has released it.

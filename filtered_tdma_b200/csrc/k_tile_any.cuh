@@ -155,6 +155,7 @@ tile_any_kernel(const __grid_constant__ AnyMaps maps, const __grid_constant__ An
     const int cid = CLUSTER ? (int)blockIdx.x / cl : (int)blockIdx.x;
     const int ncid = CLUSTER ? (int)gridDim.x / cl : (int)gridDim.x;
     const size_t ns = (size_t)args.n_sys;
+    const unsigned zero = (unsigned)args.n_sys >> 31;  // see loads_done
     // this thread's rows of every system it takes
     int r0, mlen;
     if constexpr (ASYNC) {
@@ -247,18 +248,20 @@ tile_any_kernel(const __grid_constant__ AnyMaps maps, const __grid_constant__ An
             cp_async_wait<ANY_ASYNC_NST - 2>();
         else if (ok)
             ok = mbar_wait_bounded_spin(&full[slot], phase, args.status);
+        unsigned bits = 0;
 #pragma unroll
         for (int r = 0; r < RPS; ++r) {
-            a2[r] = (double)st[0 * RPS * cols + r * rstep];
-            b2[r] = (double)st[1 * RPS * cols + r * rstep];
-            c2[r] = (double)st[2 * RPS * cols + r * rstep];
-            d2[r] = (double)st[3 * RPS * cols + r * rstep];
+            a2[r] = st[0 * RPS * cols + r * rstep];
+            b2[r] = st[1 * RPS * cols + r * rstep];
+            c2[r] = st[2 * RPS * cols + r * rstep];
+            d2[r] = st[3 * RPS * cols + r * rstep];
+            bits ^= word_of(a2[r]) ^ word_of(b2[r]) ^ word_of(c2[r]) ^ word_of(d2[r]);
         }
         if constexpr (ASYNC) {
             request();  // into the slot read one stage ago
         } else {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[slot]);
+            const unsigned z = loads_done(bits, zero);
+            if (lane == 0) mbar_arrive(&empty[slot] + z);
             // one stage later the warp whose turn it is refills the slot of stage
             // t - 1 with stage t - 1 + nst, once every warp has released it
             const int ps = slot == 0 ? nst - 1 : slot - 1;

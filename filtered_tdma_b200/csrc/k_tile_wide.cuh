@@ -287,6 +287,7 @@ tile_wide_kernel(const __grid_constant__ std::conditional_t<GEN, WideMapsGen, Wi
     const int s = tid % SYS;
     const int q = tid / SYS;
     const size_t ns = (size_t)args.n_sys;
+    const unsigned zero = (unsigned)args.n_sys >> 31;  // see loads_done
     const int c = CLUSTER ? (int)cg::this_cluster().block_rank() : 0;
     const int cid = CLUSTER ? (int)blockIdx.x / cl : (int)blockIdx.x;
     const int ncid = CLUSTER ? (int)gridDim.x / cl : (int)gridDim.x;
@@ -386,23 +387,27 @@ tile_wide_kernel(const __grid_constant__ std::conditional_t<GEN, WideMapsGen, Wi
     // release of the slot and, one stage later, its refill.
     auto fetch = [&](double (&a2)[RPS], double (&b2)[RPS], double (&c2)[RPS], double (&d2)[RPS]) {
         if (ok) ok = mbar_wait_bounded_spin(&full[slot], phase, args.status);
+        unsigned bits = 0;
 #pragma unroll
         for (int r = 0; r < RPS; ++r) {
-            a2[r] = (double)st[0 * fstep + r * rstep];
-            b2[r] = (double)st[1 * fstep + r * rstep];
-            c2[r] = (double)st[2 * fstep + r * rstep];
-            d2[r] = (double)st[3 * fstep + r * rstep];
+            const TIN va = st[0 * fstep + r * rstep], vb = st[1 * fstep + r * rstep];
+            const TIN vc = st[2 * fstep + r * rstep], vd = st[3 * fstep + r * rstep];
+            bits ^= word_of(va) ^ word_of(vb) ^ word_of(vc) ^ word_of(vd);
+            a2[r] = (double)va;
+            b2[r] = (double)vb;
+            c2[r] = (double)vc;
+            d2[r] = (double)vd;
         }
-        __syncwarp();
+        const unsigned z = loads_done(bits, zero);
         if constexpr (GEN) {
-            if (lane == 0) mbar_arrive(&empty[slot]);
+            if (lane == 0) mbar_arrive(&empty[slot] + z);
             if (warp == tw && t >= 1 && t - 1 + nst < total) {
                 if (ok) ok = mbar_wait_bounded_spin(&empty[pslot], pphase, args.status);
                 if (ok) issue(t - 1 + nst);
                 __syncwarp();
             }
         } else if (lane == 0) {
-            mbar_arrive(&empty[slot]);
+            mbar_arrive(&empty[slot] + z);
             if (t >= 1 && warp == tw && t - 1 + nst < total && ok) {
                 ok = mbar_wait_bounded_spin(&empty[pslot], pphase, args.status);
                 if (ok) issue(t - 1 + nst);

@@ -1,0 +1,33 @@
+"""Repeated solves return the same bits on every ring-fed kernel: a slot given back
+before its loads have completed shows as rare runs that differ (right after a back
+substitution's stores, on a loaded memory system)."""
+import pytest
+
+from filtered_tdma_b200 import Solver
+from filtered_tdma_b200 import _lib as L
+from filtered_tdma_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n_sys,n_row,P,cyclic,f32", [
+    (65536, 512, 8, False, False), (65536, 512, 8, False, True), (20000, 250, 4, False, False),
+    (22585, 512, 8, False, False), (4096, 2048, 16, False, False), (40000, 192, 4, True, False),
+    (2048, 128, 4, False, False)])
+def test_repeated_solves_bit_identical(cuda, n_sys, n_row, P, cyclic, f32):
+    import torch
+    dt = torch.float32 if f32 else torch.float64
+    arrays = [x.to(dt) for x in W.diag_dominant(n_sys, n_row, seed=4, device=cuda)]
+    s = Solver("pascal", n_sys, n_row, P, precision=L.FP32_STORE if f32 else L.FP64)
+    X = torch.empty((n_row, n_sys), dtype=torch.float64, device=cuda)
+    flush = torch.empty(1 << 25, dtype=torch.float64, device=cuda)
+    first = None
+    for i in range(40):
+        X.zero_()
+        if i % 4 == 0:
+            flush.fill_(i)
+        (s.solve_f32 if f32 else s.solve_out)(*arrays, X, cyclic=cyclic)
+        if first is None:
+            first = X.clone()
+        assert torch.equal(X, first)
+    assert s.status() == 0
