@@ -16,7 +16,7 @@ import sys
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 LIB = os.path.join(PKG, "libbtdma.so")
-SOURCES = [os.path.join(PKG, "csrc", f) for f in ("btdma_api.cu", "btdma_any.cu", "btdma_wide.cu",
+SOURCES = [os.path.join(PKG, "csrc", f) for f in ("btdma_api.cu", "btdma_any.cu", "btdma_wide.cu", "btdma_sh.cu",
                                                   "btdma_ragged.cu", "btdma_apps.cu")]
 DEPS = SOURCES + [os.path.join(PKG, "csrc", f) for f in os.listdir(os.path.join(PKG, "csrc"))] + [
     os.path.join(ROOT, "include", "btdma.h")]

@@ -34,17 +34,46 @@ struct btdma_heat {
 
 namespace {
 
-// One step as a kernel sequence on stream st (no host sync): right-hand side,
-// then per direction a solve with generated coefficients and the re-layout
-// for the next direction.  ev (optional): 8 events recorded around the phases
-// (the profiled step).
+// One step as a kernel sequence on stream st (no host sync): the Z, Y and X sweeps,
+// each storing its solution in the layout of the next one (X: into theta), with the
+// right-hand side formed in the Z sweep and the Y and X wall terms in theirs.  Grids
+// with an axis longer than the shared-matrix sweeps take (512 rows) run the older
+// kernels for it: the right-hand side, wall folds and transposes as passes of their
+// own.  ev (optional): 8 events recorded around the phases (the profiled step).
 int heat_enqueue(btdma_heat_t h, double* theta, cudaStream_t st, cudaEvent_t* ev = nullptr) {
     const HeatGeom& g = h->g;
     auto mark = [&](int i) {
         if (ev) cudaEventRecord(ev[i], st);
     };
-    // constant-coefficient sweep of D into X, stored through the layout map
-    // (xblk, xbs, xss, xrs) of the tiled solve (xblk = 0: X in D's layout)
+    // sweep of n_sys systems of n_row rows through the layout map (xblk, xbs, xss,
+    // xrs); wall != 0: the wall terms wall * ca[s % wblk + 1] * cb[s / wblk + 1]
+    auto shared = [&](int mode, int dir, const double* D, double* X, int n_sys, int n_row,
+                      int xblk, int xbs, int xss, int xrs, double wall, int wblk,
+                      const double* ca, const double* cb) {
+        ShArgs a = {};
+        a.X = X;
+        a.gtab = h->tab + dir * h->tab_stride;
+        a.n_sys = n_sys;
+        a.n_row = n_row;
+        a.xblk = xblk;
+        a.xbs = xbs;
+        a.xss = xss;
+        a.xrs = xrs;
+        a.wall = wall;
+        a.wblk = wblk;
+        a.ca = ca;
+        a.cb = cb;
+        a.cc = h->cosz;
+        a.fblk = g.ix;
+        a.iy = g.iy;
+        a.bx = g.bx;
+        a.by = g.by;
+        a.bz = g.bz;
+        a.src = g.dt * 3.0 * HEAT_PI * HEAT_PI;
+        a.status = h->status;
+        return try_sh(mode, D, g.ix, g.iy, a, false, st);
+    };
+    // the same sweep on the general kernel (axes above 512 rows)
     auto sweep = [&](int dir, const double* D, double* X, int n_sys, int n_row, double base,
                      int xblk, int xbs, int xss, int xrs, const char* name) {
         TileArgs ga = {};
@@ -59,67 +88,54 @@ int heat_enqueue(btdma_heat_t h, double* theta, cudaStream_t st, cudaEvent_t* ev
         return rc == 1 ? BTDMA_OK
                        : (rc < 0 ? rc : fail(BTDMA_ERR_UNSUPPORTED, "%s sweep not tileable", name));
     };
-    const dim3 b1(128, 1, 1), gr((g.ix + 127) / 128, g.iy, g.iz), bt(HEAT_TILE, 8, 1);
-    const int tx = (g.ix + HEAT_TILE - 1) / HEAT_TILE, ty = (g.iy + HEAT_TILE - 1) / HEAT_TILE;
+    const dim3 b1(128, 1, 1);
     int rc;
     mark(0);
-    if (tile_plan_heat_z(g.iz).sys != 0) {
-        // Z sweep with the right-hand side computed inside the solve from
-        // theta (no right-hand-side pass); system jj * ix + ii, row kk;
-        // solution to [jj][kk][ii]
-        mark(1);
-        TileArgs za = {};
-        za.cs = g.bz;
-        za.cbound = 1;
-        za.xblk = g.ix;
-        za.xbs = g.iz * g.ix;
-        za.xss = 1;
-        za.xrs = g.ix;
-        za.ga = h->cosx;
-        za.gb = h->cosy;
-        za.gc = h->cosz;
-        za.glam = h->hpar;
-        rc = try_heat_z(theta, h->buf1, g.ix, g.iy, g.iz, za, h->status, st, h->tab);
-        if (rc != 1) return rc < 0 ? rc : fail(BTDMA_ERR_UNSUPPORTED, "Z sweep not tileable");
-    } else {
+    // Z sweep: system jj * ix + ii, row kk; solution to [jj][kk][ii]
+    mark(1);
+    rc = shared(SH_HEAT, 0, theta, h->buf1, g.ix * g.iy, g.iz, g.ix, g.iz * g.ix, 1, g.ix, 0.0, 1,
+                h->cosx, h->cosy);
+    if (rc < 0) return rc;
+    if (rc == 0) {
+        if (g.iz <= 32 * TILE_MT)
+            return fail(BTDMA_ERR_UNSUPPORTED, "Z sweep: theta must be 16-byte aligned");
         heat_rhs_z_kernel<<<dim3((g.ix + 127) / 128, g.iy, (g.iz + HEAT_KCH - 1) / HEAT_KCH), b1,
                             0, st>>>(theta, h->buf0, g);
         CK(cudaGetLastError());
         mark(1);
-        // Z sweep: system jj * ix + ii, row kk; solution to [jj][kk][ii]
         if ((rc = sweep(0, h->buf0, h->buf1, g.ix * g.iy, g.iz, g.bz, g.ix, g.iz * g.ix, 1, g.ix,
                         "Z")))
             return rc;
     }
     mark(2);
-    heat_y_fold_kernel<<<dim3((g.ix + 127) / 128, 2, g.iz), b1, 0, st>>>(theta, h->buf1, g);
-    CK(cudaGetLastError());
     mark(3);
-    if (tile_plan(g.iy, false, 8, 1, true, true).sys != 0) {
-        // Y sweep: system kk * ix + ii, row jj; the solution goes straight into
-        // the X sweep's layout [ii][kk][jj] (rows contiguous: staged and stored
-        // coalesced), then the X wall folds on its two wall planes
+    // Y sweep: system kk * ix + ii, row jj; solution to [ii][kk][jj]
+    rc = shared(SH_ROWS, 1, h->buf1, h->buf0, g.ix * g.iz, g.iy, g.ix, g.iy, g.iz * g.iy, 1,
+                -2.0 * g.by, g.ix, h->cosx, h->cosz);
+    if (rc < 0) return rc;
+    if (rc == 0) {
+        heat_y_fold_kernel<<<dim3((g.ix + 127) / 128, 2, g.iz), b1, 0, st>>>(theta, h->buf1, g);
+        CK(cudaGetLastError());
         if ((rc = sweep(1, h->buf1, h->buf0, g.ix * g.iz, g.iy, g.by, g.ix, g.iy, g.iz * g.iy, 1,
                         "Y")))
             return rc;
-        mark(4);
-        heat_x_fold_kernel<<<dim3((g.iy + 127) / 128, 2, g.iz), b1, 0, st>>>(theta, h->buf0, g);
-    } else {
-        if ((rc = sweep(1, h->buf1, h->buf1, g.ix * g.iz, g.iy, g.by, 0, 0, 0, 0, "Y")))
-            return rc;
-        mark(4);
-        heat_y_to_x_kernel<<<dim3(tx, ty, g.iz), bt, 0, st>>>(theta, h->buf1, h->buf0, g);
     }
-    CK(cudaGetLastError());
+    mark(4);
     mark(5);
-    // X sweep: system kk * iy + jj, row ii; the solution goes straight into
-    // theta's interior (update_theta_kernel's copy, solve_theta.cu:335-347):
-    // a system's rows are contiguous there, so the sweep stages them in shared
-    // memory and stores them coalesced
+    // X sweep: system kk * iy + jj, row ii; solution to theta's interior
+    // (update_theta_kernel's copy, solve_theta.cu:335-347)
     const int plane = (g.ix + 2) * (g.iy + 2);
-    if ((rc = sweep(2, h->buf0, theta + plane + (g.ix + 2) + 1, g.iy * g.iz, g.ix, g.bx, g.iy,
-                    plane, g.ix + 2, 1, "X")))
-        return rc;
+    double* const inner = theta + plane + (g.ix + 2) + 1;
+    rc = shared(SH_ROWS, 2, h->buf0, inner, g.iy * g.iz, g.ix, g.iy, plane, g.ix + 2, 1,
+                -2.0 * g.bx, g.iy, h->cosy, h->cosz);
+    if (rc < 0) return rc;
+    if (rc == 0) {
+        heat_x_fold_kernel<<<dim3((g.iy + 127) / 128, 2, g.iz), b1, 0, st>>>(theta, h->buf0, g);
+        CK(cudaGetLastError());
+        if ((rc = sweep(2, h->buf0, inner, g.iy * g.iz, g.ix, g.bx, g.iy, plane, g.ix + 2, 1,
+                        "X")))
+            return rc;
+    }
     mark(6);
     mark(7);
     return BTDMA_OK;
@@ -637,12 +653,28 @@ int mom_tile_sweep(btdma_momentum_t h, int dir, int comp, const double* D, doubl
     if (!ready && !capturing) key.valid = false;  // rebuilt below
     const bool cyc = dir < 2 && h->pbc[dir] != 0;
     int rc;
+    if (!ready && n[dir] <= 32 * TILE_MT) {
+        rc = cyc ? build_gen_table<3, true>(n[dir], t, gt, stream)
+                 : build_gen_table<3, false>(n[dir], t, gt, stream);
+        if (rc) return rc;
+    }
+    ShArgs a = {};
+    a.X = X;
+    a.gtab = gt;
+    a.n_sys = n_sys;
+    a.n_row = n[dir];
+    a.xblk = xblk;
+    a.xbs = xbs;
+    a.xss = xss;
+    a.xrs = xrs;
+    a.fblk = g.nx;
+    a.pin = zfield && comp == 2 ? 1 : 0;
+    a.status = h->status;
+    rc = try_sh(zfield ? SH_FIELD : SH_ROWS, zfield ? zfield : D, g.nx, g.ny, a, cyc, stream);
     if (zfield) {
-        rc = try_mom_z(zfield, X, g.nx, g.ny, g.nz, t, comp == 2 ? 1 : 0, h->status, stream, gt,
-                       ready);
         if (taken) *taken = rc == 1;
         if (rc == 0) return BTDMA_OK;  // the caller gathers instead
-    } else {
+    } else if (rc == 0) {
         rc = cyc ? try_tile_gen<3, true>(D, X, n_sys, n[dir], t, h->status, stream, gt, ready)
                  : try_tile_gen<3, false>(D, X, n_sys, n[dir], t, h->status, stream, gt, ready);
     }

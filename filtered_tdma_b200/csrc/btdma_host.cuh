@@ -18,6 +18,7 @@
 #include "btdma_common.cuh"
 #include "k_segment.cuh"
 #include "k_tile.cuh"
+#include "k_tile_sh.cuh"
 #include "k_tile_wide.cuh"
 
 using namespace btdma;
@@ -41,6 +42,11 @@ int tile_wide_gen(const TIN* A, const TIN* B, const TIN* C, const TIN* D, double
 // (btdma_any.cu).  Returns as tile_solve_batch.
 int tile_any_solve(const double* A, const double* B, const double* C, const double* D, double* X,
                    int n_sys, int n_row, unsigned* status, cudaStream_t st);
+
+// A shared-matrix sweep (btdma_sh.cu): `a` without its plan fields; src is D
+// [n_row][n_sys] (SH_ROWS) or the ghosted field of nx x ny cells a plane.  Returns as
+// tile_solve_batch.
+int try_sh(int mode, const double* src, int nx, int ny, ShArgs a, bool cyclic, cudaStream_t st);
 
 struct btdma_handle {
     int method, P, precision, flags;
@@ -252,7 +258,6 @@ inline int num_sms() {
 // Shape plan of the tiled kernel: systems per group, CTAs per cluster, ring stages.
 struct TilePlan {
     int sys = 0, cl = 0, nst = 0, nseg = 0;
-    int pr = 1;  // sub-segments per thread (2: shared-matrix sweeps of 18..32 sub-segments)
 };
 
 inline int max_smem_per_sm() {
@@ -267,32 +272,15 @@ inline int max_smem_per_sm() {
     return v;
 }
 
-// na: arrays per ring stage (4, or 1 for the constant-coefficient D-only ring).
-// sh: shared-matrix sweep (factor table and lane table in shared memory).
-// tstore: the sweep stores rows contiguously through a shared tile (xrs == 1).
-inline TilePlan tile_plan(int n_row, bool cyclic, int elem = 8, int na = 4, bool sh = false,
-                          bool tstore = false) {
+// na: arrays per ring stage (4, or 1 for the generated coefficients' D-only ring).
+// sh: shared-matrix sweep (factor table in shared memory).
+inline TilePlan tile_plan(int n_row, bool cyclic, int elem = 8, int na = 4, bool sh = false) {
     TilePlan pl;
     if (n_row % TILE_MT != 0) return pl;
     const int nseg = n_row / TILE_MT;
     if (cyclic && (nseg & (nseg - 1)) != 0) return pl;  // periodic PCR needs 2^k rows
-    int sys, cl = 0, pr = 1;
-    if (sh && nseg > 16 && nseg <= 32 && nseg % 2 == 0) {
-        // Longer shared-matrix sweeps: two sub-segments per thread, so a CTA of
-        // 16 systems has at most 256 threads and two share an SM, as for the
-        // shorter sweeps below.
-        sys = 16;
-        cl = 1;
-        pr = 2;
-    } else if (sh && nseg <= 16) {
-        // Shared-matrix sweeps of up to 16 sub-segments: CTAs of at most
-        // TILE_SH_THREADS threads, two or more per SM, so that one CTA's reduced
-        // solve overlaps another's sweeps.  (Longer systems keep one CTA of up
-        // to 512 threads: splitting them over a 2-CTA cluster was measured
-        // slower, the cluster barriers waiting for the partner CTA.)
-        sys = std::min(128, TILE_SH_THREADS / tile_lanes(nseg));
-        cl = 1;
-    } else if (nseg <= 4) {
+    int sys, cl = 0;
+    if (nseg <= 4) {
         sys = 128;
         cl = 1;
     } else if (nseg <= 8) {
@@ -315,26 +303,20 @@ inline TilePlan tile_plan(int n_row, bool cyclic, int elem = 8, int na = 4, bool
     }
     int nst = na == 4 ? TILE_MAX_NST : TILE_MAX_NST_CONST;
     size_t cap = (size_t)max_smem_optin();
-    if (sh) {  // an equal share of the SM per resident CTA (128 registers a thread)
-        const int per_sm = std::max(1, 65536 / (sys * (nseg / cl / pr) * 128));
-        cap = std::min(cap, (size_t)max_smem_per_sm() / per_sm - 1024);
-    }
-    while (nst >= 3 && tile_smem_bytes(sys, nseg / cl, nseg, sys / cl, nst, elem, na, sh, 0,
-                                       tstore && cl == 1 ? n_row / pr : 0) > cap)
+    while (nst >= 3 && tile_smem_bytes(sys, nseg / cl, nseg, sys / cl, nst, elem, na, sh) > cap)
         --nst;
     if (nst < 3) return pl;
     pl.sys = sys;
     pl.cl = cl;
     pl.nst = nst;
     pl.nseg = nseg;
-    pl.pr = pr;
     return pl;
 }
 
 template <int SYS, bool CYCLIC, typename TIN = double, typename TC = double, int GEN = 0,
-          int PR = 1, bool FILT = false>
+          bool FILT = false>
 int launch_tile_sys(const CUtensorMap* maps, const TileArgs& a, cudaStream_t st) {
-    auto kern = tile_f64_kernel<SYS, CYCLIC, TIN, TC, GEN, PR, FILT>;
+    auto kern = tile_f64_kernel<SYS, CYCLIC, TIN, TC, GEN, FILT>;
     static bool attr_done = false;
     if (!attr_done) {
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -342,18 +324,11 @@ int launch_tile_sys(const CUtensorMap* maps, const TileArgs& a, cudaStream_t st)
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         attr_done = true;
     }
-    const int threads = SYS * a.nseg / a.cl / PR;
-    if (PR > 1 && (a.nseg > 32 || a.cl != 1 || (a.nseg / a.cl) % PR != 0))
-        return fail(BTDMA_ERR_UNSUPPORTED, "%d sub-segments per thread need one CTA of <= 32",
-                    PR);
+    const int threads = SYS * a.nseg / a.cl;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(threads, 1, 1);
-    constexpr bool SHT = GEN == 1 || GEN == 3 || GEN == 4 || GEN == 5;
-    // the kernel stages row-contiguous stores (xrs == 1) in a tile after the mbarriers
-    const bool tstore = SHT && a.xblk > 0 && a.xrs == 1 && a.cl == 1;
     cfg.dynamicSmemBytes = tile_smem_bytes(SYS, a.nseg / a.cl, a.nseg, SYS / a.cl, a.nst,
-                                           (int)sizeof(TIN), GEN ? 1 : 4, SHT, GEN,
-                                           tstore ? a.n_row / PR : 0);
+                                           (int)sizeof(TIN), GEN ? 1 : 4, GEN == 1 || GEN == 3);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -387,14 +362,14 @@ template <typename TIN, typename TC, bool FILT = false>
 int launch_tile_plan(const TilePlan& pl, const CUtensorMap* maps, const TileArgs& a, bool cyclic,
                      cudaStream_t st) {
     switch (pl.sys * 2 + (cyclic ? 1 : 0)) {
-        case 256: return launch_tile_sys<128, false, TIN, TC, 0, 1, FILT>(maps, a, st);
-        case 257: return launch_tile_sys<128, true, TIN, TC, 0, 1, FILT>(maps, a, st);
-        case 128: return launch_tile_sys<64, false, TIN, TC, 0, 1, FILT>(maps, a, st);
-        case 129: return launch_tile_sys<64, true, TIN, TC, 0, 1, FILT>(maps, a, st);
-        case 64: return launch_tile_sys<32, false, TIN, TC, 0, 1, FILT>(maps, a, st);
-        case 65: return launch_tile_sys<32, true, TIN, TC, 0, 1, FILT>(maps, a, st);
-        case 33: return launch_tile_sys<16, true, TIN, TC, 0, 1, FILT>(maps, a, st);
-        default: return launch_tile_sys<16, false, TIN, TC, 0, 1, FILT>(maps, a, st);
+        case 256: return launch_tile_sys<128, false, TIN, TC, 0, FILT>(maps, a, st);
+        case 257: return launch_tile_sys<128, true, TIN, TC, 0, FILT>(maps, a, st);
+        case 128: return launch_tile_sys<64, false, TIN, TC, 0, FILT>(maps, a, st);
+        case 129: return launch_tile_sys<64, true, TIN, TC, 0, FILT>(maps, a, st);
+        case 64: return launch_tile_sys<32, false, TIN, TC, 0, FILT>(maps, a, st);
+        case 65: return launch_tile_sys<32, true, TIN, TC, 0, FILT>(maps, a, st);
+        case 33: return launch_tile_sys<16, true, TIN, TC, 0, FILT>(maps, a, st);
+        default: return launch_tile_sys<16, false, TIN, TC, 0, FILT>(maps, a, st);
     }
 }
 
@@ -569,21 +544,19 @@ int try_tile(const TIN* A, const TIN* B, const TIN* C, const TIN* D, double* X, 
 template <int GEN, bool CYC = false>
 int build_gen_table(int n_row, const TileArgs& gen, double* tab, cudaStream_t st) {
     static_assert(GEN == 1 || GEN == 3, "shared-matrix modes only");
-    const TilePlan pl = tile_plan(n_row, CYC, 8, 1, true);
-    if (pl.sys == 0) return fail(BTDMA_ERR_UNSUPPORTED, "%d rows are not tileable", n_row);
+    if (n_row % TILE_MT != 0) return fail(BTDMA_ERR_UNSUPPORTED, "%d rows are not tileable", n_row);
     if (!tab) return fail(BTDMA_ERR_ARG, "shared-matrix sweep without a factor table");
     TileArgs a = gen;
     a.n_row = n_row;
-    a.nseg = pl.nseg;
-    a.cl = pl.cl;
-    a.nst = pl.nst;
-    tile_table_kernel<GEN, CYC><<<(pl.nseg + 127) / 128, 128, 0, st>>>(a, tab);
+    a.nseg = n_row / TILE_MT;
+    tile_table_kernel<GEN, CYC><<<(a.nseg + 127) / 128, 128, 0, st>>>(a, tab);
     CK(cudaGetLastError());
     return BTDMA_OK;
 }
 
 // Generated-coefficient batch, only D read (the GEN modes of the tiled
-// kernel; the coefficient fields of `gen` are used, the rest is filled here).
+// kernel; GEN 1 and 3 for systems above 32 sub-segments, which k_tile_sh.cuh does not
+// take; the coefficient fields of `gen` are used, the rest is filled here).
 // Returns 1 when launched, 0 when the shape is not tiled, < 0 on error.
 // GEN 1 and 3 (one matrix for every system): `tab` is device scratch of
 // gen_table_doubles(n_row) doubles for the shared elimination factors, built
@@ -592,8 +565,7 @@ template <int GEN, bool CYC = false>
 int try_tile_gen(const double* D, double* X, int n_sys, int n_row, const TileArgs& gen,
                  unsigned* status, cudaStream_t st, double* tab = nullptr,
                  bool table_ready = false) {
-    const bool tstore = (GEN == 1 || GEN == 3) && gen.xblk > 0 && gen.xrs == 1;
-    const TilePlan pl = tile_plan(n_row, CYC, 8, 1, GEN == 1 || GEN == 3, tstore);
+    const TilePlan pl = tile_plan(n_row, CYC, 8, 1, GEN == 1 || GEN == 3);
     if (pl.sys == 0 || !tma_ok_elem(D, n_sys, 8)) return 0;
     const int nsc = pl.nseg / pl.cl;
     CUtensorMap maps[4];
@@ -617,11 +589,10 @@ int try_tile_gen(const double* D, double* X, int n_sys, int n_row, const TileArg
         a.gtab = tab;
     }
     int rc;
-    if constexpr (GEN == 1 || GEN == 3) {
-        if (pl.pr == 2) {
-            rc = launch_tile_sys<16, CYC, double, double, GEN, 2>(maps, a, st);
-            return rc == BTDMA_OK ? 1 : rc;
-        }
+    if constexpr (GEN == 1 || GEN == 3) {  // above 32 sub-segments: 16 systems a cluster
+        if (pl.sys != 16) return 0;
+        rc = launch_tile_sys<16, CYC, double, double, GEN>(maps, a, st);
+        return rc == BTDMA_OK ? 1 : rc;
     }
     switch (pl.sys) {
         case 128: rc = launch_tile_sys<128, CYC, double, double, GEN>(maps, a, st); break;
@@ -629,166 +600,6 @@ int try_tile_gen(const double* D, double* X, int n_sys, int n_row, const TileArg
         case 32: rc = launch_tile_sys<32, CYC, double, double, GEN>(maps, a, st); break;
         default: rc = launch_tile_sys<16, CYC, double, double, GEN>(maps, a, st); break;
     }
-    return rc == BTDMA_OK ? 1 : rc;
-}
-
-// Heat Z sweep with the right-hand side fused (GEN 4 of the tiled kernel):
-// the plan (16 systems per group, one CTA of 16 x n_row / 16 threads, 2 to 32
-// sub-segments), or sys == 0 when the shape does not take it.
-inline TilePlan tile_plan_heat_z(int n_row) {
-    TilePlan pl;
-    if (n_row % TILE_MT != 0) return pl;
-    const int nseg = n_row / TILE_MT;
-    if (nseg < 2 || nseg > 32) return pl;
-    // one sub-segment per thread: with two, the stencil's stage values and the
-    // two recurrences exceed 128 registers and spill
-    const int pr = 1;
-    const int T = TILE_HEAT_SYS * nseg / pr;
-    const int per_sm = std::max(1, 65536 / (T * 128));
-    const size_t cap = std::min((size_t)max_smem_optin(), (size_t)max_smem_per_sm() / per_sm - 1024);
-    int nst = TILE_MAX_NST_CONST;
-    while (nst >= 2 &&
-           tile_smem_bytes(TILE_HEAT_SYS, nseg, nseg, TILE_HEAT_SYS, nst, 8, 1, true, 4) > cap)
-        --nst;
-    if (nst < 2) return pl;
-    pl.sys = TILE_HEAT_SYS;
-    pl.cl = 1;
-    pl.nst = nst;
-    pl.nseg = nseg;
-    pl.pr = pr;
-    return pl;
-}
-
-// 4-D view of the heat field theta [(iz + 2) x (iy + 2) x (ix + 2)] for the
-// fused Z sweep: (x = i, y = j, row within the sub-segment, sub-segment) from
-// plane k = 1; boxes of TILE_HEAT_BOX_I x 3 x 4 rows x nsc sub-segments.
-inline bool make_heat_theta_map(CUtensorMap* map, const double* theta, int ix, int iy, int nseg,
-                                int nsc) {
-    auto fn = encode_fn();
-    if (!fn) return false;
-    const size_t nx = (size_t)ix + 2, plane = nx * ((size_t)iy + 2);
-    cuuint64_t dims[4] = {(cuuint64_t)nx, (cuuint64_t)iy + 2, (cuuint64_t)TILE_MT,
-                          (cuuint64_t)nseg};
-    cuuint64_t strides[3] = {nx * sizeof(double), plane * sizeof(double),
-                             (cuuint64_t)TILE_MT * plane * sizeof(double)};
-    cuuint32_t box[4] = {(cuuint32_t)TILE_HEAT_BOX_I, 3u, (cuuint32_t)tile_rps(8, 1),
-                         (cuuint32_t)nsc};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<double*>(theta + plane),
-                    dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS;
-}
-
-// The heat Z sweep with its right-hand side computed inside the solve from
-// theta (GEN 4).  gen carries the sweep's fields: cs = bz, cbound = 1, ga / gb
-// / gc = cos(pi x), cos(pi y), cos(pi z) tables (ghosts included), glam = the
-// device array {bx, by, dt 3 pi^2, iy, iz}, xblk = ix and the output layout map.
-// tab: the Z matrix's factor table (build_gen_table<1>).  Returns 1 when
-// launched, 0 when the shape is not taken, < 0 on error.
-inline int try_heat_z(const double* theta, double* X, int ix, int iy, int iz, const TileArgs& gen,
-                      unsigned* status, cudaStream_t st, const double* tab) {
-    const TilePlan pl = tile_plan_heat_z(iz);
-    if (pl.sys == 0 || ix % TILE_HEAT_SYS != 0 ||
-        (reinterpret_cast<uintptr_t>(theta) & 15) != 0 || ((size_t)(ix + 2) * 8) % 16 != 0)
-        return 0;
-    CUtensorMap maps[4];
-    if (!make_heat_theta_map(&maps[3], theta, ix, iy, pl.nseg, pl.nseg)) return 0;
-    maps[0] = maps[1] = maps[2] = maps[3];  // not read in this mode
-    TileArgs a = gen;
-    a.X = X;
-    a.n_sys = ix * iy;
-    a.n_row = iz;
-    a.nseg = pl.nseg;
-    a.cl = pl.cl;
-    a.nst = pl.nst;
-    a.n_groups = a.n_sys / TILE_HEAT_SYS;
-    a.status = status;
-    a.gtab = tab;
-    const int rc = launch_tile_sys<TILE_HEAT_SYS, false, double, double, 4>(maps, a, st);
-    return rc == BTDMA_OK ? 1 : rc;
-}
-
-// Momentum z sweep reading the ghosted field directly (GEN 5 of the tiled
-// kernel): 16 systems per group, two sub-segments per thread above 16
-// sub-segments (as tile_plan's shared-matrix sweeps), or sys == 0.
-inline TilePlan tile_plan_field_z(int n_row) {
-    TilePlan pl;
-    if (n_row % TILE_MT != 0) return pl;
-    const int nseg = n_row / TILE_MT;
-    if (nseg < 2 || nseg > 32) return pl;
-    const int pr = nseg > 16 && nseg % 2 == 0 ? 2 : 1;
-    const int T = TILE_HEAT_SYS * nseg / pr;
-    const int per_sm = std::max(1, 65536 / (T * 128));
-    const size_t cap = std::min((size_t)max_smem_optin(), (size_t)max_smem_per_sm() / per_sm - 1024);
-    int nst = TILE_MAX_NST_CONST;
-    while (nst >= 3 &&
-           tile_smem_bytes(TILE_HEAT_SYS, nseg, nseg, TILE_HEAT_SYS, nst, 8, 1, true, 5) > cap)
-        --nst;
-    if (nst < 3) return pl;
-    pl.sys = TILE_HEAT_SYS;
-    pl.cl = 1;
-    pl.nst = nst;
-    pl.nseg = nseg;
-    pl.pr = pr;
-    return pl;
-}
-
-// 4-D view of a ghosted field q [(nz + 2) x (ny + 2) x (nx + 2)] for the z
-// sweep: (x = i, y = j, row within the sub-segment, sub-segment) from plane
-// k = 1; boxes of TILE_HEAT_BOX_I x 1 x 4 rows x nsc sub-segments.
-inline bool make_field_row_map(CUtensorMap* map, const double* q, int nx, int ny, int nseg,
-                               int nsc) {
-    auto fn = encode_fn();
-    if (!fn) return false;
-    const size_t rx = (size_t)nx + 2, plane = rx * ((size_t)ny + 2);
-    cuuint64_t dims[4] = {(cuuint64_t)rx, (cuuint64_t)ny + 2, (cuuint64_t)TILE_MT,
-                          (cuuint64_t)nseg};
-    cuuint64_t strides[3] = {rx * sizeof(double), plane * sizeof(double),
-                             (cuuint64_t)TILE_MT * plane * sizeof(double)};
-    cuuint32_t box[4] = {(cuuint32_t)TILE_HEAT_BOX_I, 1u, (cuuint32_t)tile_rps(8, 1),
-                         (cuuint32_t)nsc};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<double*>(q + plane), dims,
-                    strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS;
-}
-
-// The momentum z sweep straight from the ghosted field q (no gather): system
-// s = (j - 1) nx + (i - 1), row k - 1; x through gen's layout map (xblk = nx).
-// gen carries the GEN 3 row tables (ga, gb, gc), cs and the map; pin: row 0 is
-// x = 0 (the w component).  tab: the (z, comp) factor table, built here unless
-// table_ready.  Returns 1 when launched, 0 when the shape is not taken, < 0 on
-// error.
-inline int try_mom_z(const double* q, double* X, int nx, int ny, int nz, const TileArgs& gen,
-                     int pin, unsigned* status, cudaStream_t st, double* tab, bool table_ready) {
-    const TilePlan pl = tile_plan_field_z(nz);
-    if (pl.sys == 0 || nx % TILE_HEAT_SYS != 0 || (reinterpret_cast<uintptr_t>(q) & 15) != 0 ||
-        ((size_t)(nx + 2) * 8) % 16 != 0 || gen.xblk != nx)
-        return 0;
-    CUtensorMap maps[4];
-    if (!make_field_row_map(&maps[3], q, nx, ny, pl.nseg, pl.nseg)) return 0;
-    maps[0] = maps[1] = maps[2] = maps[3];  // not read in this mode
-    TileArgs a = gen;
-    a.X = X;
-    a.n_sys = nx * ny;
-    a.n_row = nz;
-    a.nseg = pl.nseg;
-    a.cl = pl.cl;
-    a.nst = pl.nst;
-    a.n_groups = a.n_sys / TILE_HEAT_SYS;
-    a.status = status;
-    a.gpin = pin;
-    if (!table_ready) {
-        tile_table_kernel<3, false><<<(pl.nseg + 127) / 128, 128, 0, st>>>(a, tab);
-        CK(cudaGetLastError());
-    }
-    a.gtab = tab;
-    const int rc = pl.pr == 2
-                       ? launch_tile_sys<TILE_HEAT_SYS, false, double, double, 5, 2>(maps, a, st)
-                       : launch_tile_sys<TILE_HEAT_SYS, false, double, double, 5>(maps, a, st);
     return rc == BTDMA_OK ? 1 : rc;
 }
 

@@ -18,20 +18,12 @@
 //     kernels write there;
 //   * A, B, C are never materialised (the solve generates them);
 //   * the right-hand side of the step (all directions' explicit half and the
-//     Z wall folds) is computed inside the Z sweep from theta (the tiled
-//     solve's GEN 4 mode, k_tile.cuh), so it is never stored; heat_rhs_z_kernel
-//     below remains for Z sweeps that mode does not take (fewer than 2 or
-//     more than 32 sub-segments);
-//   * the Z sweep stores its solution straight into the Y sweep's layout
-//     ([kk][jj][ii] -> [jj][kk][ii], the tiled solve's mapped store; the Y wall
-//     folds then touch the two wall planes only), and the X sweep straight
-//     into theta (its rows are contiguous there: the tiled solve stages each
-//     group's solution in shared memory and stores it coalesced; storing it
-//     row by row from the lanes, rows 2 KB apart, was slower than a separate
-//     transpose); the Y sweep stores into the X sweep's layout the same way,
-//     and the X wall folds touch the two wall planes.  heat_y_to_x_kernel
-//     (a transpose through shared-memory tiles) remains for Y sweeps whose
-//     staged store does not fit.
+//     Z wall folds) is computed inside the Z sweep from theta, and the Y and X wall
+//     terms inside their sweeps (k_tile_sh.cuh), so a step is three kernels;
+//   * each sweep stores its solution in the next one's layout: Z ([kk][jj][ii]) in
+//     the Y sweep's [jj][kk][ii], Y in the X sweep's [ii][kk][jj], X in theta.
+// Axes longer than those sweeps take (512 rows) run the kernels below: the
+// right-hand side and the wall terms as passes of their own.
 #pragma once
 
 #include "btdma_common.cuh"
@@ -138,8 +130,7 @@ __global__ void __launch_bounds__(128) heat_y_fold_kernel(const double* __restri
 
 // X wall folds on the Y solution, already in the X-sweep layout [ii][kk][jj]
 // (build_lhs_x_kernel's right-hand-side terms, solve_theta.cu:256-332): planes
-// ii = 0 and ii = ix - 1 get base * (ghost + boundary cell), added to the
-// value as heat_y_to_x_kernel adds it.  Grid (iy / 128, 2, iz).
+// ii = 0 and ii = ix - 1 get base * (ghost + boundary cell).  Grid (iy / 128, 2, iz).
 __global__ void __launch_bounds__(128) heat_x_fold_kernel(const double* __restrict__ theta,
                                                           double* __restrict__ Dx,
                                                           const HeatGeom g) {
@@ -151,42 +142,6 @@ __global__ void __launch_bounds__(128) heat_x_fold_kernel(const double* __restri
     const double t = theta[heat_full(g, i, j, k)];
     const double ubc = -g.cy[j] * g.cz[k];
     Dx[((size_t)ii * g.iz + kk) * g.iy + jj] += g.bx * ((2.0 * ubc - t) + t);
-}
-
-constexpr int HEAT_TILE = 32;
-
-// Y solution [jj][kk][ii] -> X-sweep layout [ii][kk][jj] plus the X wall folds
-// (copy_y_to_rhs + build_lhs_x_kernel, solve_theta.cu:256-332), through a
-// shared 32 x 32 tile so both sides are coalesced.  Block (32, 8).
-__global__ void __launch_bounds__(256) heat_y_to_x_kernel(const double* __restrict__ theta,
-                                                          const double* __restrict__ Dy,
-                                                          double* __restrict__ Dx,
-                                                          const HeatGeom g) {
-    __shared__ double tile[HEAT_TILE][HEAT_TILE + 1];
-    const int ii0 = blockIdx.x * HEAT_TILE, jj0 = blockIdx.y * HEAT_TILE, kk = blockIdx.z;
-#pragma unroll
-    for (int u = 0; u < HEAT_TILE / 8; ++u) {  // block (HEAT_TILE, 8)
-        const int r = threadIdx.y + 8 * u;
-        const int ii = ii0 + threadIdx.x, jj = jj0 + r;
-        if (ii < g.ix && jj < g.iy) tile[r][threadIdx.x] = Dy[((size_t)jj * g.iz + kk) * g.ix + ii];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < HEAT_TILE / 8; ++u) {  // block (HEAT_TILE, 8)
-        const int r = threadIdx.y + 8 * u;
-        const int jj = jj0 + threadIdx.x, ii = ii0 + r;
-        if (ii < g.ix && jj < g.iy) {
-            double v = tile[threadIdx.x][r];
-            if (ii == 0 || ii == g.ix - 1) {
-                const int j = jj + 1, k = kk + 1, i = ii == 0 ? 1 : g.ix;
-                const double t = theta[heat_full(g, i, j, k)];
-                const double ubc = -g.cy[j] * g.cz[k];
-                if (ii == 0) v += g.bx * ((2.0 * ubc - t) + t);
-                if (ii == g.ix - 1) v += g.bx * ((2.0 * ubc - t) + t);
-            }
-            Dx[((size_t)ii * g.iz + kk) * g.iy + jj] = v;
-        }
-    }
 }
 
 // Initial field on the full grid, ghosts included (mpi_subdomain.cpp

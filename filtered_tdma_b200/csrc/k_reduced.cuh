@@ -392,4 +392,55 @@ __device__ __forceinline__ void reduced_solve_rhs(double r0, double r1, int p, i
     xf = r0 - lt[3 * ls] * xlm - lt[4 * ls] * xl;
 }
 
+// reduced_solve_rhs for two systems a lane (r0, r1 hold the first / last rows' values
+// of both): the table entries are read once, and the two chains fill each other's
+// latency.
+template <bool CYCLIC>
+__device__ __forceinline__ void reduced_solve_rhs2(double2 r0, double2 r1, int p, int nseg, int W,
+                                                   const double* __restrict__ lt, int ls,
+                                                   double& xf0, double& xl0, double& xf1,
+                                                   double& xl1) {
+    const unsigned FULL = 0xffffffffu;
+    const int pn = ((CYCLIC && p == nseg - 1) ? 0 : p + 1) & (W - 1);
+    const double na = __shfl_sync(FULL, r0.x, pn, W), nb = __shfl_sync(FULL, r0.y, pn, W);
+    double ra, rb;
+    {
+        const double l1 = lt[1 * ls], u1 = lt[2 * ls], ib = lt[0];
+        ra = (r1.x - l1 * r0.x - u1 * na) * ib;
+        rb = (r1.y - l1 * r0.y - u1 * nb) * ib;
+    }
+    if (CYCLIC && nseg == 1) {
+        ra *= lt[7 * ls];
+        rb *= lt[7 * ls];
+    } else {
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            const int dl = 1 << v;
+            if (dl >= nseg) break;
+            int im = p - dl, ip = p + dl;
+            if (CYCLIC) {
+                im = im < 0 ? im + nseg : im;
+                ip = ip >= nseg ? ip - nseg : ip;
+            }
+            im &= W - 1;
+            ip &= W - 1;
+            const double ma = __shfl_sync(FULL, ra, im, W), mb = __shfl_sync(FULL, rb, im, W);
+            const double pa = __shfl_sync(FULL, ra, ip, W), pb = __shfl_sync(FULL, rb, ip, W);
+            const double l = lt[(5 + 3 * v) * ls], u = lt[(6 + 3 * v) * ls];
+            const double ib = lt[(7 + 3 * v) * ls];
+            ra = (ra - l * ma - u * pa) * ib;
+            rb = (rb - l * mb - u * pb) * ib;
+            if (CYCLIC && 2 * dl == nseg) break;
+        }
+    }
+    const int pm = ((CYCLIC && p == 0) ? nseg - 1 : p - 1) & (W - 1);
+    double ma = __shfl_sync(FULL, ra, pm, W), mb = __shfl_sync(FULL, rb, pm, W);
+    if (!CYCLIC && p == 0) ma = mb = 0.0;
+    const double l0 = lt[3 * ls], u0 = lt[4 * ls];
+    xl0 = ra;
+    xl1 = rb;
+    xf0 = r0.x - l0 * ma - u0 * ra;
+    xf1 = r0.y - l0 * mb - u0 * rb;
+}
+
 }  // namespace btdma

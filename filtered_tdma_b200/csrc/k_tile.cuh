@@ -62,7 +62,6 @@ __host__ __device__ constexpr int tile_rps(int elem, int na = 4) {
     return (na == 1 ? 32 : 16) / elem;
 }
 constexpr int TILE_MAX_THREADS = 512;
-constexpr int TILE_SH_THREADS = 256;  // CTA size limit of the shared-matrix sweeps
 constexpr int TILE_MAX_NST = 8;       // ring stages (upper bound)
 constexpr int TILE_MAX_NST_CONST = 16;  // ring stages of D-only (constant-coefficient) rings
 
@@ -109,13 +108,8 @@ struct TileArgs {
         // Generated-coefficient modes (GEN != 0) may store x through a layout
         // map instead of the plain [n_row][n_sys]: with xblk > 0, row j of
         // system s goes to  X + (s / xblk) * xbs + (s % xblk) * xss + j * xrs
-        // (xrs > 0).  The heat step writes its Z sweep in the Y sweep's layout
-        // and its X sweep into the ghosted field, without a copy pass.  xrs == 1
-        // (a system's rows contiguous) in a shared-matrix sweep of one CTA per
-        // group stages the group's x in shared memory and stores every
-        // system's rows with coalesced warp stores (the launch adds the tile,
-        // tile_tstore_bytes).  (A union with the refinement fields: a larger
-        // argument struct made ptxas spill more in every instantiation.)
+        // (xrs > 0).  (A union with the refinement fields: a larger argument
+        // struct made ptxas spill more in every instantiation.)
         struct {
             int xblk, xbs, xss, xrs;
         };
@@ -137,8 +131,8 @@ struct TileArgs {
     const double* gb;
     const double* gc;
     const double* glam;
-    // GEN 1 and 3: every system of the batch has the same matrix, so the
-    // elimination of each sub-segment is computed once (tile_table_kernel) into
+    // GEN 1 and 3 (longer systems than k_tile_sh.cuh takes): every system of the
+    // batch has the same matrix, so the elimination of each sub-segment is computed once (tile_table_kernel) into
     // gtab: per row [inv pivot, a * inv, pi, alpha, gamma] (n_row x 5), then
     // per sub-segment [r, r c0, l0, u0, l1, u1] (nseg x 6), then (up to 32
     // sub-segments) the reduced system's lane table at tile_red_offset(n_row);
@@ -182,56 +176,27 @@ __host__ __device__ __forceinline__ size_t tile_fixed_doubles(int sys, int nsc, 
     return f;
 }
 // Elements of one ring stage: na arrays of RPS rows of sys systems of nsc
-// sub-segments; GEN == 4 (heat Z sweep with the right-hand side fused): a box of
-// theta of TILE_HEAT_BOX_I x 3 cells (the 16 systems' columns with their x
-// and y neighbours) per row instead of one D value per system.
-constexpr int TILE_HEAT_SYS = 16;
-constexpr int TILE_HEAT_BOX_I = TILE_HEAT_SYS + 2;
-// GEN == 5 (momentum z sweep reading the ghosted field): one row of 18 cells.
-// tile_stage_box_elems: what a stage's TMA boxes deliver (its transaction
-// count); tile_stage_elems: the distance between stages, rounded up to 128
-// bytes, since a tensor copy's shared-memory destination must be 128-byte
-// aligned (the 18-cell boxes of GEN 4 / 5 are not, for an odd nsc).
-__host__ __device__ __forceinline__ int tile_stage_box_elems(int sys, int nsc, int elem, int na,
-                                                             int gen = 0) {
-    return gen == 4   ? TILE_HEAT_BOX_I * 3 * tile_rps(elem, na) * nsc
-           : gen == 5 ? TILE_HEAT_BOX_I * tile_rps(elem, na) * nsc
-                      : na * tile_rps(elem, na) * sys * nsc;
-}
-__host__ __device__ __forceinline__ int tile_stage_elems(int sys, int nsc, int elem, int na,
-                                                         int gen = 0) {
-    const int b = tile_stage_box_elems(sys, nsc, elem, na, gen);
-    if (gen != 4 && gen != 5) return b;  // rows of SYS systems: whole 128-byte multiples
-    const int q = 128 / elem;
-    return (b + q - 1) / q * q;
+// sub-segments.
+__host__ __device__ __forceinline__ int tile_stage_elems(int sys, int nsc, int elem, int na) {
+    return na * tile_rps(elem, na) * sys * nsc;
 }
 // na: arrays per ring stage (4: A, B, C, D; 1: D only).
 __host__ __device__ __forceinline__ size_t tile_ring_bytes(int sys, int nsc, int nst, int elem,
-                                                           int na = 4, int gen = 0) {
-    return (size_t)nst * tile_stage_elems(sys, nsc, elem, na, gen) * elem;
+                                                           int na = 4) {
+    return (size_t)nst * tile_stage_elems(sys, nsc, elem, na) * elem;
 }
 // Shared-matrix table slice of one CTA (its nsc sub-segments): per row 5 and
 // per sub-segment 6 doubles.
 __host__ __device__ __forceinline__ size_t tile_tab_doubles(int nsc) {
     return (size_t)nsc * TILE_MT * 5 + (size_t)nsc * 6;
 }
-// Row-contiguous stores (xrs == 1): a [sys][rows + 1] tile of x after the
-// mbarriers, rows = n_row / PR (a thread owning two sub-segments stages and
-// stores the group's two halves in turn); the odd pitch keeps the back
-// substitution's writes, 16 systems a warp, on distinct banks.
-__host__ __device__ __forceinline__ size_t tile_tstore_bytes(int sys, int rows) {
-    return (size_t)sys * (rows + 1) * sizeof(double);
-}
 __host__ __device__ __forceinline__ size_t tile_smem_bytes(int sys, int nsc, int nseg, int sub,
                                                            int nst, int elem = 8, int na = 4,
-                                                           bool shared_tab = false, int gen = 0,
-                                                           int tstore_rows = 0) {
-    return tile_ring_bytes(sys, nsc, nst, elem, na, gen) +
+                                                           bool shared_tab = false) {
+    return tile_ring_bytes(sys, nsc, nst, elem, na) +
            (shared_tab ? tile_tab_doubles(nsc) * sizeof(double) : 0) +
            tile_fixed_doubles(sys, nsc, nseg, sub, shared_tab) * sizeof(double) +
-           (gen == 4 ? ((size_t)nseg * TILE_MT + 2) * sizeof(double) : 0) +
-           2ull * nst * sizeof(uint64_t) + 128 +
-           (tstore_rows > 0 ? tile_tstore_bytes(sys, tstore_rows) : 0);
+           2ull * nst * sizeof(uint64_t) + 128;
 }
 
 __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, int x, int y,
@@ -274,16 +239,11 @@ __device__ __forceinline__ void tile_cluster_sync(int cl) {
 // 3, were measured at two CTAs per SM as well: at 64 registers a thread they
 // spill and run 1.5x the instructions, which costs more than the second CTA
 // hides.)
-// PR: sub-segments per thread.  The shared-matrix sweeps keep only delta per
-// row, so a thread can own two sub-segments (ql and ql + nsc / 2): half the
-// threads per system, two independent recurrences per thread, and CTAs small
-// enough that two share an SM and one's reduced solve overlaps the other's
-// streaming.
 // FILT: the reduced system takes Filtered's 2 x 2 interfaces between segments
 // of R = (mode >> TILE_MODE_FILT_SHIFT) sub-segments (a separate
 // instantiation: the extra paths would cost the exact kernels registers).
 template <int SYS, bool CYCLIC, typename TIN = double, typename TC = double, int GEN = 0,
-          int PR = 1, bool FILT = false>
+          bool FILT = false>
 __global__ void __launch_bounds__(TILE_MAX_THREADS, 1)
 tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                 const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmD,
@@ -292,10 +252,7 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     constexpr int M = TILE_MT;
     constexpr bool CONSTC = GEN != 0;                 // coefficients generated, D only
     // one matrix for all systems (gtab)
-    constexpr bool SH = GEN == 1 || GEN == 3 || GEN == 4 || GEN == 5;
-    static_assert(GEN != 4 || (SYS == TILE_HEAT_SYS && !CYCLIC), "heat Z sweep: 16 systems");
-    static_assert(GEN != 5 || (SYS == TILE_HEAT_SYS && !CYCLIC), "field-box sweep: 16 systems");
-    static_assert(PR == 1 || (PR == 2 && SH), "two sub-segments per thread: shared matrix only");
+    constexpr bool SH = GEN == 1 || GEN == 3;
     static_assert(!FILT || GEN == 0, "Filtered interfaces: matrices read from A, B, C");
     constexpr int NA = CONSTC ? 1 : 4;                // arrays per ring stage
     constexpr int RPS = tile_rps((int)sizeof(TIN), NA);  // rows per ring stage
@@ -304,9 +261,7 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     extern __shared__ unsigned char smem_raw[];
     const int nseg = args.nseg, cl = args.cl, nst = args.nst;
     const int nsc = nseg / cl;   // sub-segments per CTA
-    const int hsc = nsc / PR;    // thread rows: a thread owns sub-segments ql + h * hsc
-    const int TS = SYS * nsc;    // columns of a ring stage
-    const int T = SYS * hsc;     // == blockDim.x
+    const int T = SYS * nsc;     // == blockDim.x
     const int sub = SYS / cl;    // systems whose reduced system this CTA solves
     const int W = tile_lanes(nseg);
     const bool shuffled = W <= 32;
@@ -315,21 +270,16 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
     TIN* ring = reinterpret_cast<TIN*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-    const int sstride = tile_stage_elems(SYS, nsc, (int)sizeof(TIN), NA, GEN);  // per stage
+    const int sstride = tile_stage_elems(SYS, nsc, (int)sizeof(TIN), NA);  // per stage
     double* red = reinterpret_cast<double*>(ring + (size_t)nst * sstride);
     double* xr = red + (rhs_red ? 2 : 6) * fstride;
     double* pcr = xr + 2 * fstride;  // only when !shuffled
     const int gs = nseg + 2;
     double* tabs = pcr + (shuffled ? 0 : 6 * gs * sub);  // SH: this CTA's factor table
     double* lanes = tabs + (SH ? tile_tab_doubles(nsc) : 0);  // rhs_red: lane table [k][p]
-    // GEN == 4: the cos(pi z) table of the rows (ghosts included), read every row
-    double* czt = lanes + (rhs_red ? 32 * TILE_RED_LANE : 0);
-    uint64_t* full = reinterpret_cast<uint64_t*>(czt + (GEN == 4 ? args.n_row + 2 : 0));
+    uint64_t* full =
+        reinterpret_cast<uint64_t*>(lanes + (rhs_red ? 32 * TILE_RED_LANE : 0));
     uint64_t* empty = full + nst;
-    // row-contiguous stores through a shared tile (shared-matrix modes, one CTA)
-    const bool tstore = SH && args.xblk > 0 && args.xrs == 1 && cl == 1;
-    double* xt = reinterpret_cast<double*>(empty + nst);  // [SYS][n_row / PR + 1] when tstore
-    const int xtp = args.n_row / PR + 1;
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -362,8 +312,6 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             for (int i = threadIdx.x; i < 32 * TILE_RED_LANE; i += blockDim.x)
                 lanes[(i % TILE_RED_LANE) * 32 + i / TILE_RED_LANE] = g2[i];
         }
-        if constexpr (GEN == 4)
-            for (int i = threadIdx.x; i < args.n_row + 2; i += blockDim.x) czt[i] = args.gc[i];
     }
     if (!shuffled && tid < sub) {  // zero guard rows of the PCR buffers
         for (int f = 0; f < 6; ++f) {
@@ -386,11 +334,7 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                          ? (args.n_groups - cluster_id + n_clusters - 1) / n_clusters
                          : 0;
     const int total = n_my * SPG;  // ring stages this CTA consumes
-    // bytes the TMA boxes of a stage deliver (the 18-cell boxes' stride is padded)
-    const uint32_t stage_bytes =
-        (GEN == 4 || GEN == 5)
-            ? (uint32_t)tile_stage_box_elems(SYS, nsc, (int)sizeof(TIN), NA, GEN) * sizeof(TIN)
-            : (uint32_t)sstride * sizeof(TIN);
+    const uint32_t stage_bytes = (uint32_t)sstride * sizeof(TIN);
 
     auto issue = [&](int t) {  // one thread
         const int slot = t % nst;
@@ -398,21 +342,6 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const int k0 = (t % SPG) * RPS;
         TIN* dst = ring + (size_t)slot * sstride;
         mbar_expect_tx(&full[slot], stage_bytes);
-        if constexpr (GEN == 4) {
-            // theta box: x from the system's left neighbour (ghosted index ii0),
-            // y = jj - 1 .. jj + 1 (ghosted jj .. jj + 2), RPS rows of every
-            // sub-segment (the map's base is plane k = 1)
-            const int s0 = g * SYS;
-            tma_load_4d(dst, &tmD, s0 % args.xblk, s0 / args.xblk, k0, c * nsc, &full[slot]);
-            return;
-        }
-        if constexpr (GEN == 5) {
-            // the field's row (x from the system's left neighbour, ghosted
-            // index ii0; y = jj + 1), RPS rows of every sub-segment
-            const int s0 = g * SYS;
-            tma_load_4d(dst, &tmD, s0 % args.xblk, s0 / args.xblk + 1, k0, c * nsc, &full[slot]);
-            return;
-        }
         if constexpr (!CONSTC) {
             tma_load_3d(dst + 0 * RPS * T, &tmA, g * SYS, k0, c * nsc, &full[slot]);
             tma_load_3d(dst + 1 * RPS * T, &tmB, g * SYS, k0, c * nsc, &full[slot]);
@@ -441,158 +370,28 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const bool valid = sys < args.n_sys;
 
         // ------------------------------------------------------ forward pass
-        // rows 1..M-1 used (register resident); deP[h]: sub-segment ql + h * hsc
-        TC al[M], ga[M], deP[PR][M];
-        TC db0P[PR], sdP[PR];
-#pragma unroll
-        for (int h = 0; h < PR; ++h) db0P[h] = sdP[h] = 0;
-        TC(&de)[M] = deP[0];  // the one sub-segment of the PR == 1 modes
-        TC& db0 = db0P[0];
-        TC& sd = sdP[0];
+        TC al[M], ga[M], de[M];  // rows 1..M-1 used (register resident)
+        TC db0 = 0, sd = 0;
         double lam = 0.0;  // GEN == 2: this system's diagonal shift
         if constexpr (GEN == 2) lam = valid ? args.glam[sys >> 1] : 0.0;
         TC ab0 = 0, cb0 = 0;
         TC pi = 1, sa = 0;
-        if constexpr (GEN == 4) {
-            // Heat Z sweep: the right-hand side of every row is computed here
-            // from the theta box of the stage (the reference's rhs_kernel and
-            // build_lhs_z wall folds, apps/heat_gpu/solve_theta.cu:121-202),
-            // with the ghosts computed where read (2 u_BC - theta).  Row k's z
-            // neighbours are rows k - 1 and k + 1, so a row is finished one row
-            // later; row 0 of the sub-segment takes its lower neighbour from the
-            // previous sub-segment's last row in the last stage, row M - 1 its
-            // upper one from the next sub-segment's first row in the first.
-            const double* hp = args.glam;  // bx, by, dt 3 pi^2, iy, iz
-            const int ixg = args.xblk, s0 = g * SYS;
-            const int jj = s0 / ixg, ii = s0 % ixg + s;
-            const int iy = (int)__ldg(hp + 3), iz = (int)__ldg(hp + 4);
-            const double bx = __ldg(hp + 0), by = __ldg(hp + 1), bz = args.cs,
-                         srcs = __ldg(hp + 2);
-            const double cxi = __ldg(args.ga + ii + 1), cyj = __ldg(args.gb + jj + 1);
-            const double diag = 1.0 + (-2.0 * bx) + (-2.0 * by) + (-2.0 * bz);
-            const double ubz = -cxi * cyj;
-            const double sxy = srcs * cxi * cyj;  // the source term's x, y factor
-            // per owned sub-segment: row 0's partial sum, the pending row's
-            // partial sum, the previous row's theta, the neighbours' edge rows
-            double pp0[PR], pp[PR], pc[PR], tnext[PR], tkm0[PR];
-#pragma unroll
-            for (int h = 0; h < PR; ++h) pp0[h] = pp[h] = pc[h] = tnext[h] = tkm0[h] = 0.0;
-            // the recurrence of the shared-matrix modes on a finished row
-            auto feed = [&](int h, int k, double d) {
-                const double* tr = tabs + ((ql + h * hsc) * M + k) * 5;
-                if (k == 1) {
-                    deP[h][1] = d * tr[0];
-                    sdP[h] = deP[h][1];
-                } else {
-                    deP[h][k] = d * tr[0] - tr[1] * deP[h][k - 1];
-                    if (k <= M - 2) sdP[h] += tr[2] * deP[h][k];
-                }
-            };
+        {
 #pragma unroll
             for (int j = 0; j < SPG; ++j) {
                 if (ok) ok = mbar_wait_bounded(&full[slot], phase, args.status);
-                // box [sub-segment][row][y][x], x = system + 1 (+-1: x neighbours)
-                const double* sb = ring + (size_t)slot * sstride;
-                auto at = [&](int qq, int r, int y, int dx) {
-                    return sb[((qq * RPS + r) * 3 + y) * TILE_HEAT_BOX_I + s + 1 + dx];
-                };
-#pragma unroll
-                for (int h = 0; h < PR; ++h) {
-                    const int qq = ql + h * hsc;  // sub-segment in the CTA
-                    const int q = c * nsc + qq;
-                    const int kk0 = q * M;
-                    if (j == 0 && q + 1 < nseg) tnext[h] = at(qq + 1, 0, 1, 0);
-                    if (j == SPG - 1 && q > 0) tkm0[h] = at(qq - 1, RPS - 1, 1, 0);
-                    double tc[RPS], tl[RPS], tr_[RPS], ym[RPS], yp[RPS];
-#pragma unroll
-                    for (int r = 0; r < RPS; ++r) {
-                        tc[r] = at(qq, r, 1, 0);
-                        tl[r] = at(qq, r, 1, -1);
-                        tr_[r] = at(qq, r, 1, 1);
-                        ym[r] = at(qq, r, 0, 0);
-                        yp[r] = at(qq, r, 2, 0);
-                    }
-#pragma unroll
-                    for (int r = 0; r < RPS; ++r) {
-                        const int k = j * RPS + r;
-                        const int kk = kk0 + k;
-                        const double tt = tc[r];
-                        const double czk = czt[kk + 1];
-                        const double ux = -cyj * czk, uy = -cxi * czk;  // x, y wall values
-                        const double tip = ii + 1 < ixg ? tr_[r] : 2.0 * ux - tt;
-                        const double tim = ii > 0 ? tl[r] : 2.0 * ux - tt;
-                        const double tjp = jj + 1 < iy ? yp[r] : 2.0 * uy - tt;
-                        const double tjm = jj > 0 ? ym[r] : 2.0 * uy - tt;
-                        const double src = sxy * czk;
-                        double p =
-                            (bx * tip + bx * tim) + (by * tjp + by * tjm) + diag * tt + src;
-                        if (kk == 0) p += bz * (2.0 * ubz - tt) + bz * ((2.0 * ubz - tt) + tt);
-                        if (kk == iz - 1)
-                            p += bz * (2.0 * ubz - tt) + bz * ((2.0 * ubz - tt) + tt);
-                        if (k >= 1) p += bz * pc[h];  // lower neighbour: the previous row
-                        if (k == 1) pp0[h] += bz * tt;  // row 0's upper neighbour
-                        if (k >= 2) feed(h, k - 1, pp[h] + bz * tt);
-                        if (k == 0)
-                            pp0[h] = p;
-                        else
-                            pp[h] = p;
-                        pc[h] = tt;
-                    }
-                    // PR == 2: one sub-segment's stage values live at a time
-                    if constexpr (PR == 2) __syncwarp();
-                }
-                {  // release the slot (after the arithmetic: measured spill-free)
-                    __syncwarp();
-                    if (lane == 0) {
-                        mbar_arrive(&empty[slot]);
-                        if (t >= 1 && warp == tw && t - 1 + nst < total && ok) {
-                            ok = mbar_wait_bounded(&empty[pslot], pphase, args.status);
-                            if (ok) issue(t - 1 + nst);
-                        }
-                    }
-                    pslot = slot;
-                    pphase = phase;
-                    ++t;
-                    if (++tw == nwarps) tw = 0;
-                    if (++slot == nst) {
-                        slot = 0;
-                        phase ^= 1u;
-                    }
-                }
-            }
-            // row M - 1: the next sub-segment's first row above it            // row M - 1: the next sub-segment's first row above it (the top wall's
-            // ghost is already in); row 0: the previous sub-segment's last row
-            // below it (or the bottom wall's ghost, already in)
-#pragma unroll
-            for (int h = 0; h < PR; ++h) {
-                const int qq = ql + h * hsc;
-                const int kk0 = (c * nsc + qq) * M;
-                feed(h, M - 1, kk0 + M - 1 == iz - 1 ? pp[h] : pp[h] + bz * tnext[h]);
-                db0P[h] = (kk0 == 0 ? pp0[h] : pp0[h] + bz * tkm0[h]) * tabs[(qq * M) * 5];
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < SPG; ++j) {
-                if (ok) ok = mbar_wait_bounded(&full[slot], phase, args.status);
-                TIN a2[RPS], b2[RPS], c2[RPS], d2[PR][RPS];  // widened where used
+                TIN a2[RPS], b2[RPS], c2[RPS], d2[RPS];  // widened where used
                 unsigned bits = 0;
 #pragma unroll
                 for (int r = 0; r < RPS; ++r) {
                     if constexpr (!CONSTC) {
-                        a2[r] = st[0 * RPS * TS + r * SYS];
-                        b2[r] = st[1 * RPS * TS + r * SYS];
-                        c2[r] = st[2 * RPS * TS + r * SYS];
+                        a2[r] = st[0 * RPS * T + r * SYS];
+                        b2[r] = st[1 * RPS * T + r * SYS];
+                        c2[r] = st[2 * RPS * T + r * SYS];
+                        bits ^= word_of(a2[r]) ^ word_of(b2[r]) ^ word_of(c2[r]);
                     }
-#pragma unroll
-                    for (int h = 0; h < PR; ++h) {
-                        if constexpr (GEN == 5)  // box [sub-segment][row][x], x = system + 1
-                            d2[h][r] = ring[(size_t)slot * sstride +
-                                            ((ql + h * hsc) * RPS + r) * TILE_HEAT_BOX_I + s + 1];
-                        else
-                            d2[h][r] = st[(NA - 1) * RPS * TS + h * hsc * RPS * SYS + r * SYS];
-                        bits ^= word_of(d2[h][r]);
-                    }
-                    if constexpr (!CONSTC) bits ^= word_of(a2[r]) ^ word_of(b2[r]) ^ word_of(c2[r]);
+                    d2[r] = st[(NA - 1) * RPS * T + r * SYS];
+                    bits ^= word_of(d2[r]);
                 }
                 const unsigned z = loads_done(bits, zero);
                 if (lane == 0) {
@@ -617,32 +416,25 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
                 if constexpr (SH) {  // right-hand side only, factors from gtab
 #pragma unroll
-                    for (int h = 0; h < PR; ++h)
-#pragma unroll
-                        for (int r = 0; r < RPS; ++r) {
-                            const int k = j * RPS + r;
-                            const double* tr = tabs + ((ql + h * hsc) * M + k) * 5;
-                            double d = (double)d2[h][r];
-                            // GEN == 5 with gpin: row 0 of the system is x = 0
-                            // (the w component's first face, k_build_z)
-                            if (GEN == 5 && args.gpin != 0 && c * nsc + ql + h * hsc == 0 &&
-                                k == 0)
-                                d = 0.0;
-                            if (k == 0) {
-                                db0P[h] = d * tr[0];
-                            } else if (k == 1) {
-                                deP[h][1] = d * tr[0];
-                                sdP[h] = deP[h][1];
-                            } else {
-                                deP[h][k] = d * tr[0] - tr[1] * deP[h][k - 1];
-                                if (k <= M - 2) sdP[h] += tr[2] * deP[h][k];
-                            }
+                    for (int r = 0; r < RPS; ++r) {
+                        const int k = j * RPS + r;
+                        const double* tr = tabs + (ql * M + k) * 5;
+                        const double d = (double)d2[r];
+                        if (k == 0) {
+                            db0 = d * tr[0];
+                        } else if (k == 1) {
+                            de[1] = d * tr[0];
+                            sd = de[1];
+                        } else {
+                            de[k] = d * tr[0] - tr[1] * de[k - 1];
+                            if (k <= M - 2) sd += tr[2] * de[k];
                         }
+                    }
                 } else {
 #pragma unroll
                     for (int r = 0; r < RPS; ++r) {
                         const int k = j * RPS + r;
-                        TC a, b, cc, d = (TC)d2[0][r];
+                        TC a, b, cc, d = (TC)d2[r];
                         if constexpr (GEN == 2) {
                             const int kg = (c * nsc + ql) * M + k;  // row of the system
                             const double ta = args.ga[kg], tc = args.gc[kg];
@@ -689,22 +481,18 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
         // reduced rows of this sub-segment -> red[f][ql][s]
         if constexpr (SH) {
-#pragma unroll
-            for (int h = 0; h < PR; ++h) {
-                const int qq = ql + h * hsc;
-                const double* sb = tabs + nsc * M * 5 + qq * 6;
-                double* w = red + qq * RP + s;
-                if (rhs_red) {  // r0 | r1 only
-                    w[0] = sb[0] * (double)db0P[h] - sb[1] * (double)sdP[h];
-                    w[fstride] = (double)deP[h][M - 1];
-                } else {
-                    w[2 * fstride] = sb[0] * (double)db0P[h] - sb[1] * (double)sdP[h];
-                    w[5 * fstride] = (double)deP[h][M - 1];
-                    w[0 * fstride] = sb[2];
-                    w[1 * fstride] = sb[3];
-                    w[3 * fstride] = sb[4];
-                    w[4 * fstride] = sb[5];
-                }
+            const double* sb = tabs + nsc * M * 5 + ql * 6;
+            double* w = red + ql * RP + s;
+            if (rhs_red) {  // r0 | r1 only
+                w[0] = sb[0] * (double)db0 - sb[1] * (double)sd;
+                w[fstride] = (double)de[M - 1];
+            } else {
+                w[2 * fstride] = sb[0] * (double)db0 - sb[1] * (double)sd;
+                w[5 * fstride] = (double)de[M - 1];
+                w[0 * fstride] = sb[2];
+                w[1 * fstride] = sb[3];
+                w[3 * fstride] = sb[4];
+                w[4 * fstride] = sb[5];
             }
         } else {
             const TC pi_last = -ga[M - 2] * pi;
@@ -834,68 +622,47 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         tile_cluster_sync(cl);
 
         // --------------------------------------------------- back substitution
+        const double x_first = xr[ql * RP + s];
+        const double x_last = xr[fstride + ql * RP + s];
+        if (valid) {
+            const int q = c * nsc + ql;
+            double* xp = args.X + (size_t)(q * M + M - 1) * ns + sys;  // row M-1
+            if constexpr (CONSTC) {
+                if (args.xblk > 0)
+                    xp = args.X + (ptrdiff_t)(sys / args.xblk) * (ptrdiff_t)args.xbs +
+                         (ptrdiff_t)(sys % args.xblk) * (ptrdiff_t)args.xss +
+                         (size_t)(q * M + M - 1) * ns;
+            }
+            // corrections are accumulated only by the FP32 inner solve of
+            // refinement (the FP64-arithmetic instantiations keep the plain
+            // store); the old x of all M rows is loaded before any store
+            double xo[M] = {};
+            bool acc = false;
+            if constexpr (sizeof(TC) == 4) {
+                acc = (args.mode & TILE_MODE_ACCUMULATE) != 0;
+                if (acc) {
 #pragma unroll
-        for (int h = 0; h < PR; ++h) {
-            const int qq = ql + h * hsc;  // sub-segment in the CTA
-            const double x_first = xr[qq * RP + s];
-            const double x_last = xr[fstride + qq * RP + s];
-            if (valid) {
-                const int q = c * nsc + qq;
-                double* xp = args.X + (size_t)(q * M + M - 1) * ns + sys;  // row M-1
-                if constexpr (CONSTC) {
-                    if (tstore)  // staged, rows contiguous (relative to this half's first row)
-                        xp = xt + (size_t)s * xtp + ql * M + M - 1;
-                    else if (args.xblk > 0)
-                        xp = args.X + (ptrdiff_t)(sys / args.xblk) * (ptrdiff_t)args.xbs +
-                             (ptrdiff_t)(sys % args.xblk) * (ptrdiff_t)args.xss +
-                             (size_t)(q * M + M - 1) * ns;
+                    for (int k = 0; k < M; ++k)
+                        xo[k] = xp[-(ptrdiff_t)(M - 1 - k) * (ptrdiff_t)ns];
                 }
-                // corrections are accumulated only by the FP32 inner solve of
-                // refinement (the FP64-arithmetic instantiations keep the plain
-                // store); the old x of all M rows is loaded before any store
-                double xo[M] = {};
-                bool acc = false;
-                if constexpr (sizeof(TC) == 4) {
-                    acc = (args.mode & TILE_MODE_ACCUMULATE) != 0;
-                    if (acc) {
+            }
+            *xp = acc ? xo[M - 1] + x_last : x_last;
+            double xn = x_last;
 #pragma unroll
-                        for (int k = 0; k < M; ++k) xo[k] = xp[-(ptrdiff_t)(M - 1 - k) * (ptrdiff_t)ns];
-                    }
-                }
-                *xp = acc ? xo[M - 1] + x_last : x_last;
-                double xn = x_last;
-#pragma unroll
-                for (int k = M - 2; k >= 1; --k) {
-                    xp -= ns;
-                    if constexpr (SH) {
-                        const double* tr = tabs + (qq * M + k) * 5;
-                        xn = (double)deP[h][k] - tr[3] * x_first - tr[4] * xn;
-                    } else {
-                        xn = (double)de[k] - (double)al[k] * x_first - (double)ga[k] * xn;
-                    }
-                    nonfinite = fma(xn, 0.0, nonfinite);
-                    *xp = acc ? xo[k] + xn : xn;
-                }
+            for (int k = M - 2; k >= 1; --k) {
                 xp -= ns;
-                *xp = acc ? xo[0] + x_first : x_first;
-                nonfinite = fma(x_first, 0.0, fma(x_last, 0.0, nonfinite));
-            }
-            if (tstore) {
-                // this half's x from the tile, each system's rows by one warp
-                // with coalesced stores; the tile is written again after the
-                // barrier below, or after the next group's two barriers
-                const int r0 = h * hsc * M, nr = hsc * M;
-                __syncthreads();
-                for (int ss = warp; ss < SYS; ss += nwarps) {
-                    const int sg = g * SYS + ss;
-                    if (sg >= args.n_sys) break;
-                    double* dst = args.X + (ptrdiff_t)(sg / args.xblk) * (ptrdiff_t)args.xbs +
-                                  (ptrdiff_t)(sg % args.xblk) * (ptrdiff_t)args.xss + r0;
-                    const double* src = xt + (size_t)ss * xtp;
-                    for (int r = lane; r < nr; r += 32) dst[r] = src[r];
+                if constexpr (SH) {
+                    const double* tr = tabs + (ql * M + k) * 5;
+                    xn = (double)de[k] - tr[3] * x_first - tr[4] * xn;
+                } else {
+                    xn = (double)de[k] - (double)al[k] * x_first - (double)ga[k] * xn;
                 }
-                if (h + 1 < PR) __syncthreads();
+                nonfinite = fma(xn, 0.0, nonfinite);
+                *xp = acc ? xo[k] + xn : xn;
             }
+            xp -= ns;
+            *xp = acc ? xo[0] + x_first : x_first;
+            nonfinite = fma(x_first, 0.0, fma(x_last, 0.0, nonfinite));
         }
     }
     if (nonfinite != 0.0) raise_status(args.status, ST_NONFINITE);  // NaN != 0
