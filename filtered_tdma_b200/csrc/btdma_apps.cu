@@ -293,8 +293,12 @@ int btdma_heat_step(btdma_heat_t h, double* theta, int n_steps, int use_graph,
         h->exec = nullptr;
         h->graph = nullptr;
         // one uncaptured step on a zeroed scratch field first, so the kernels'
-        // first-use attribute calls stay out of the capture (theta is untouched)
+        // first-use attribute calls stay out of the capture (theta is untouched);
+        // after the caller's earlier steps, which may still use the sweep buffers
         const HeatGeom& g = h->g;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(stream, &cap));
+        if (cap == cudaStreamCaptureStatusNone) CK(cudaStreamSynchronize(stream));
         CK(cudaMemsetAsync(h->scratch, 0, sizeof(double) * (size_t)(g.ix + 2) * (g.iy + 2) *
                                               (g.iz + 2), h->cap));
         int rc = heat_enqueue(h, h->scratch, h->cap);
