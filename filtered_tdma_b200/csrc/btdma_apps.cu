@@ -7,6 +7,7 @@
 #include "btdma_host.cuh"
 #include "k_heat.cuh"
 #include "k_momentum.cuh"
+#include "k_poisson.cuh"
 
 // ------------------------------------------------------------- heat ADI step
 struct btdma_heat {
@@ -425,8 +426,65 @@ int btdma_poisson_destroy(btdma_poisson_t h) {
     return BTDMA_OK;
 }
 
+namespace {
+
+// The pair kernel (k_poisson.cuh).  1: launched, 0: not its shape, < 0: error.
+int launch_poisson(btdma_poisson_t h, double* rhs, cudaStream_t st) {
+    constexpr int M = TILE_MT;
+    auto kern = poisson_kernel;
+    static bool attr_done = false;
+    if (!attr_done) {
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                max_smem_optin()));
+        attr_done = true;
+    }
+    PoisArgs a = {};
+    a.X = rhs;
+    a.ga = h->ga;
+    a.gc = h->gc;
+    a.lam = h->lam;
+    a.nz = h->nz;
+    a.n_modes = h->n_modes;
+    a.pin = h->pin;
+    a.nseg = h->nz / M;
+    a.status = h->status;
+    // the modes that fill 256 threads (a box is at most 256 values wide), then as few
+    // as still take that many rounds
+    const int slots = num_sms();
+    int np = std::min(128, POIS_THREADS / a.nseg);
+    const int rounds = (h->n_modes + np * slots - 1) / (np * slots);
+    np = std::max(1, std::min(np, (h->n_modes + rounds * slots - 1) / (rounds * slots)));
+    if (pois_smem_bytes(np, a.nseg, h->nz) > (size_t)max_smem_optin())
+        return 0;
+    a.np = np;
+    a.n_groups = (h->n_modes + np - 1) / np;
+    auto fn = encode_fn();
+    if (!fn) return 0;
+    const size_t row = 2 * (size_t)h->n_modes * sizeof(double);
+    CUtensorMap tm;
+    cuuint64_t dims[3] = {2 * (cuuint64_t)h->n_modes, (cuuint64_t)M, (cuuint64_t)a.nseg};
+    cuuint64_t strides[2] = {row, row * M};
+    cuuint32_t boxd[3] = {2 * (cuuint32_t)np, (cuuint32_t)M, (cuuint32_t)a.nseg};
+    cuuint32_t estr[3] = {1, 1, 1};
+    if (fn(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, rhs, dims, strides, boxd, estr,
+           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return 0;
+    const int threads = (np * a.nseg + 31) / 32 * 32;
+    kern<<<std::min(slots, a.n_groups), threads, pois_smem_bytes(np, a.nseg, h->nz), st>>>(tm, a);
+    CK(cudaGetLastError());
+    return 1;
+}
+
+}  // namespace
+
 int btdma_poisson_solve(btdma_poisson_t h, double* rhs, cudaStream_t stream) {
     if (!h || !rhs) return fail(BTDMA_ERR_ARG, "null argument");
+    // up to 32 sub-segments of 16 rows; longer columns on the general tiled kernel
+    if (tma_ok(rhs, 2) && h->nz <= 32 * TILE_MT) {
+        const int rc = launch_poisson(h, rhs, stream);
+        if (rc != 0) return rc < 0 ? rc : BTDMA_OK;
+    }
     TileArgs g = {};
     g.ga = h->ga;
     g.gc = h->gc;
