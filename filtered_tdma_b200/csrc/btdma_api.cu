@@ -55,7 +55,7 @@ int jmax_launch(btdma_t h, const double* D, int n_sys, int n_row, cudaStream_t s
 // exact: the device word jfinal sets when the batch needs the exact reduced
 // solve (null: the reference's behaviour, no fallback)
 int jfinal_launch(btdma_t h, int n_row, int version, unsigned* exact, cudaStream_t st) {
-    jfinal_kernel<<<1, 32, 0, st>>>(h->work, h->J, h->rho_row, n_row, h->P, h->eps_constant,
+    jfinal_kernel<<<1, 32 * SEG_MAX_P, 0, st>>>(h->work, h->J, h->rho_row, n_row, h->P, h->eps_constant,
                                     version, (h->flags & BTDMA_FLAG_J_HOST) ? 1 : 0, exact);
     CK(cudaGetLastError());
     return BTDMA_OK;

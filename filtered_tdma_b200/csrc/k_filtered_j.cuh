@@ -63,7 +63,15 @@ jmax_kernel(const double* __restrict__ D, int n_sys, int n_row, int P, int all_r
     }
     unsigned long long bits = __double_as_longlong(v);
     for (int o = 16; o > 0; o >>= 1) bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(&work[2 * k], bits);
+    // one atomic a block (one a warp queued up on the segment's word: 11 us for 16 rows
+    // of 65536 systems)
+    __shared__ unsigned long long part[JRED_BLOCK / 32];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = bits;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < JRED_BLOCK / 32; ++w) bits = max(bits, part[w]);
+        atomicMax(&work[2 * k], bits);
+    }
 }
 
 // J per segment from the accumulated maxima; resets the accumulators.
@@ -76,17 +84,24 @@ jmax_kernel(const double* __restrict__ D, int n_sys, int n_row, int P, int all_r
 // exact (optional): set to 1 when some segment has rho >= 0.5 (the bound does
 // not hold) or J >= m - 2 (the truncation keeps every row, so only the 2x2
 // interface approximation would remain), else 0: the solve then takes the exact
-// reduced system instead of the Filtered interface.  One warp.
+// reduced system instead of the Filtered interface.  One block, a warp per segment:
+// the rows' bounds are read 32 at a time (one thread a segment read them one after
+// another: 8.3 us for 8 segments of 64 rows).
 __global__ void jfinal_kernel(unsigned long long* __restrict__ work, int* __restrict__ J,
                               const double* __restrict__ rho_row, int n_row, int P,
                               double eps_constant, int version, int host_semantics,
                               unsigned* __restrict__ exact) {
-    bool need_exact = false;
-    for (int k = threadIdx.x; k < P; k += blockDim.x) {
+    __shared__ unsigned need;
+    if (threadIdx.x == 0) need = 0u;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int k = threadIdx.x >> 5; k < P; k += blockDim.x >> 5) {  // a warp per segment
         int r0, m;
         seg_range(n_row, P, k, r0, m);
         double rho = 0.0;
-        for (int j = 1; j < m; ++j) rho = fmax(rho, rho_row[r0 + j]);
+        for (int j = 1 + lane; j < m; j += 32) rho = fmax(rho, rho_row[r0 + j]);
+        for (int o = 16; o > 0; o >>= 1) rho = fmax(rho, __shfl_xor_sync(0xffffffffu, rho, o));
+        if (lane != 0) continue;
         const double m0 = __longlong_as_double((long long)work[2 * k]);
         const double mn = __longlong_as_double((long long)work[2 * k + 1]);
         int Jk;
@@ -112,12 +127,12 @@ __global__ void jfinal_kernel(unsigned long long* __restrict__ work, int* __rest
             Jk = (int)Jl;
         }
         J[k] = Jk;
-        need_exact |= rho >= 0.5 || Jk >= m - 2;
+        if (rho >= 0.5 || Jk >= m - 2) atomicOr(&need, 1u);
         work[2 * k] = 0ull;
         work[2 * k + 1] = 0ull;
     }
-    const bool any = __any_sync(0xffffffffu, need_exact);
-    if (exact != nullptr && threadIdx.x == 0) *exact = any ? 1u : 0u;
+    __syncthreads();
+    if (exact != nullptr && threadIdx.x == 0) *exact = need;
 }
 
 }  // namespace btdma

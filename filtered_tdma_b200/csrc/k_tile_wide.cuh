@@ -260,6 +260,12 @@ tile_wide_kernel(const __grid_constant__ std::conditional_t<GEN, WideMapsGen, Wi
     constexpr int SPG = M / RPS;  // stages per group
     constexpr int RP = SYS + 1;
     constexpr bool PAD = GEN && !CYCLIC;
+    // a closed gate: nothing to do (TILE_MODE_GATE_ZERO: open while *gate == 0); every
+    // CTA reads the same word
+    if (!GEN && args.gate != nullptr &&
+        ((*static_cast<const volatile unsigned*>(args.gate) == 0u) !=
+         ((args.mode & TILE_MODE_GATE_ZERO) != 0)))
+        return;
     extern __shared__ unsigned char smem_raw[];
     const int nseg = args.nseg, nst = args.nst;  // nseg: sub-segments of this CTA
     const int cl = CLUSTER ? args.cl : 1;
@@ -315,13 +321,8 @@ tile_wide_kernel(const __grid_constant__ std::conditional_t<GEN, WideMapsGen, Wi
     const uint32_t tcol = *static_cast<volatile uint32_t*>(tslot) + ((uint32_t)(warp & 3) << 21) +
                           (uint32_t)(warp >> 2) * WIDE_TCOLS;
 
-    // a closed gate leaves the CTA without groups (TILE_MODE_GATE_ZERO: the
-    // gate is open while *gate == 0)
-    const bool gated_off = args.gate != nullptr &&
-                           ((*static_cast<const volatile unsigned*>(args.gate) == 0u) !=
-                            ((args.mode & TILE_MODE_GATE_ZERO) != 0));
     const int filt_r = FILT ? (args.mode >> TILE_MODE_FILT_SHIFT) & 255 : 0;  // lanes a segment
-    const int n_my = (!gated_off && args.n_groups > cid)
+    const int n_my = args.n_groups > cid
                          ? (args.n_groups - cid + ncid - 1) / ncid
                          : 0;
     const int total = n_my * SPG;
