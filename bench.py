@@ -736,7 +736,7 @@ def main():
             # 5 kernels a step (the sweeps' factor tables are built at
             # create): Z sweep with the right-hand side, Y wall folds, Y sweep,
             # X wall folds, X sweep
-            "launches_per_step": 5, "graph": True,
+            "launches_per_step": 3, "graph": True,
             "finite": bool(torch.isfinite(th).all().item())}
         heat.close()
         del th
@@ -855,10 +855,10 @@ def main():
             "data": "synthetic",
             "config": {"workload": WORKLOAD, "n_sys": N_SYS, "n_row": N_ROW, "P": P,
                        "method": "pascal", "per_rank_batch": True,
-                       "kernel_sub_segments": N_ROW // 16,
-                       "kernel_note": "P = 8 is the reference's rank count; the tiled "
-                                      "kernel splits every system into n_row / 16 = 32 "
-                                      "sub-segments of 16 rows and solves the 64-unknown "
+                       "kernel_sub_segments": N_ROW // 32,
+                       "kernel_note": "P = 8 is the reference's rank count; the wide "
+                                      "kernel splits every system into n_row / 32 = 16 "
+                                      "sub-segments of 32 rows and solves the 32-unknown "
                                       "reduced system exactly, so the result does not "
                                       "depend on P",
                        "cpu_baseline_sample": "16384 systems x 512 rows (1/16 of the "

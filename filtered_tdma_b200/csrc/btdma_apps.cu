@@ -827,8 +827,7 @@ int btdma_momentum_sweep(btdma_momentum_t h, int dir, int comp, const double* q,
         return mom_tile_sweep(h, 1, comp, h->buf, dst_in, g.nx, sp, 1, g.nx + 2, c, stream);
     }
     // x: system s = (k, j), j = s % ny fastest, row r -> dst(i = r + 1, j, k): a
-    // system's rows are contiguous in the field, so the sweep stages them and
-    // stores them coalesced (no transposing scatter)
+    // system's rows are contiguous in the field (no transposing scatter)
     mom_gather_x_kernel<<<dim3((g.nx + MOM_TILE - 1) / MOM_TILE, (g.ny + MOM_TILE - 1) / MOM_TILE,
                                g.nz), bt, 0, stream>>>(q, h->buf, g);
     CK(cudaGetLastError());
@@ -847,8 +846,8 @@ int btdma_momentum_adi(btdma_momentum_t h, int comp, double* rhs, double* q_out,
     }
     // Each sweep stores its solution straight into the next sweep's layout:
     // z (read from rhs itself) -> y layout [j][k][i] (mapped rows), y -> x
-    // layout [i][k][j] (contiguous rows: staged, coalesced), x -> q_out's
-    // interior (staged); rhs is only read.
+    // layout [i][k][j] (contiguous rows), x -> q_out's
+    // interior; rhs is only read.
     const MomGeom& g = h->g;
     const dim3 b1(128, 1, 1);
     const int sp = (g.nx + 2) * (g.ny + 2);

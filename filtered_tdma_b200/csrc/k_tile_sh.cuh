@@ -15,6 +15,13 @@
 //     back substitution not finite (x_k enters x_{k-1} times a finite factor, and
 //     0 x Inf is NaN), so rows 1 and 0 of a sub-segment stand for all.
 //
+// Measured on B200 (k_tile.cuh's modes before / now): heat sweeps of 256 x 384 x 512, Z
+// 339 / 286 us, Y 279 + 14 (its fold) / 185, X 199 / 140; momentum 256^3 209 / 167 for
+// the three.  Z reads 2.25 cells a cell from L2; X is at 90 % of the copy bandwidth.
+// Wider groups alone did nothing for the old modes (X 199 -> 227 us at 32 systems); rows
+// stored with single elements at their misaligned ends took X 250 us; 20 systems a group
+// for the 24 sub-segments of Y (240 threads, 160-byte pieces) 195 us.
+//
 // MODE SH_ROWS   D in the sweep's layout [n_row][n_sys]; optional wall terms on the
 //                first and last row (the heat step's fully implicit walls)
 //      SH_FIELD  rows read from a ghosted field: boxes of SYS + 2 cells
@@ -232,8 +239,9 @@ tile_sh_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ S
             }
         };
         if constexpr (MODE == SH_HEAT) {
-            // as k_tile.cuh's GEN 4: a row is finished when the one above it is read;
-            // row 0 takes its lower neighbour in the last stage, row M - 1 its upper
+            // the 7-point right-hand side (the reference's rhs_kernel and build_lhs_z,
+            // apps/heat_gpu/solve_theta.cu:121-202), ghosts computed where they are
+            // read: a row is finished when the one above it is read; row 0 takes its lower neighbour in the last stage, row M - 1 its upper
             // one in the first (from the neighbouring sub-segments' rows)
             const int ix = args.fblk;
             const double bx = args.bx, by = args.by, bz = args.bz;

@@ -361,7 +361,7 @@ int btdma_poisson_status(btdma_poisson_t h, unsigned* status, cudaStream_t strea
  * MomentumSolverGPU::advance's diffuse step after k_lap and writes the result
  * into q_out's interior.  With the default (PaScaL) backend it only reads
  * rhs: each sweep stores its solution straight into the next sweep's layout
- * (four kernels); with a Filtered backend it runs the reference's sequence, z
+ * (three kernels); with a Filtered backend it runs the reference's sequence, z
  * and y in place on rhs.  PaScaL (exact)
  * solves; n a multiple of 16, n / 16 a power of two for periodic sweeps.  The
  * handle keeps each (dir, comp) factor table until c or the stream changes;
