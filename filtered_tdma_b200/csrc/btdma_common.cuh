@@ -213,6 +213,17 @@ __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// The cluster's barrier in its .aligned form, which wants every lane of the warp at the
+// same instruction: callers may come from per-lane branches, so the warp converges here.
+__device__ __forceinline__ void cluster_arrive() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // ------------------------------------------------------------- segmentation
 // Block split of n rows into P segments (first `rem` segments one row longer),
 // the reference's para_range (libs/pascal_tdma/cpu/para_range.cpp:4-10).

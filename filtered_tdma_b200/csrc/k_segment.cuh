@@ -108,13 +108,6 @@ __host__ __device__ __forceinline__ size_t seg_smem_bytes(int mcap, int P, bool 
     return tiles + red + rsc + bars + 128;  // +128: alignment slack
 }
 
-__device__ __forceinline__ void cluster_arrive() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() {
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // RR: leading rows of each segment held in registers (when every segment has
 // at least RR + 2 rows, so rows m - 2 and m - 1 are tile rows).
 template <int METHOD, bool CYCLIC, int RR = 0>
@@ -570,7 +563,6 @@ seg_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // before this CTA's shared memory is released.
         for (int c = 0; c < nch; ++c) mbar_wait_bounded(&bars[c], 0, nullptr, 1u << 16);
     }
-    __syncwarp();
     cluster_wait();  // the neighbours are done reading this CTA's shared memory
 #undef T
 }

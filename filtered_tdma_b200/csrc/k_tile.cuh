@@ -224,8 +224,8 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 
 __device__ __forceinline__ void tile_cluster_sync(int cl) {
     if (cl > 1) {
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        cluster_arrive();
+        cluster_wait();
     } else {
         __syncthreads();
     }

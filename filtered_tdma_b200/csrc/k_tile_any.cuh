@@ -319,12 +319,7 @@ tile_any_kernel(const __grid_constant__ AnyMaps maps, const __grid_constant__ An
                 else
                     block(kb, first, false);
             };
-            auto keep = [&](int kb) {
-                __syncwarp();
-                tmem_store4(tcol + kb * 6, ta);
-                tmem_store4(tcol + kb * 6 + 8, tg);
-                tmem_store4(tcol + kb * 6 + 16, td);
-            };
+            auto keep = [&](int kb) { tmem_store_rows(tcol + kb * 6, ta, tg, td); };
             rows(0, true);
             keep(0);
 #pragma unroll 1
@@ -455,17 +450,12 @@ tile_any_kernel(const __grid_constant__ AnyMaps maps, const __grid_constant__ An
                 put(xn);
             }
         }
-        __syncwarp();
         tmem_wait_st();
 #pragma unroll
         for (int k0 = TR - 4; k0 >= 0; k0 -= 4) {
             if (k0 < m) {
                 uint32_t wa[8], wg[8], wd[8];
-                __syncwarp();
-                tmem_load4(tcol + k0 * 6, wa);
-                tmem_load4(tcol + k0 * 6 + 8, wg);
-                tmem_load4(tcol + k0 * 6 + 16, wd);
-                tmem_wait_ld(wa, wg, wd);
+                tmem_load_rows(tcol + k0 * 6, wa, wg, wd);
 #pragma unroll
                 for (int r = 3; r >= 0; --r) {
                     if (k0 + r == 0) continue;  // row 0 is x_first

@@ -107,9 +107,14 @@ __host__ __device__ __forceinline__ int wide_tmem_cols(int warps) {
     while (c < (warps + 3) / 4 * WIDE_TCOLS) c <<= 1;
     return c;
 }
+// tcgen05's .sync.aligned instructions need every lane of the warp at the same
+// instruction, and callers come from per-lane branches (stores of systems past the
+// batch, rows past a tail): each of these wrappers converges the warp itself.
+//
 // One warp; the address of the columns is written to *dst (shared memory).  The
 // call waits while another CTA on the SM holds the columns.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst, uint32_t cols) {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(dst)),
                  "r"(cols)
@@ -117,35 +122,47 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* dst, uint32_t cols) {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols)
                  : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() {
+    __syncwarp();
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
-// 4 doubles of every lane to / from 8 columns of the warp's lanes.  All lanes of
-// the warp call them together.
-__device__ __forceinline__ void tmem_store4(uint32_t addr, const double (&v)[4]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr),
-        "r"(__double2loint(v[0])), "r"(__double2hiint(v[0])), "r"(__double2loint(v[1])),
-        "r"(__double2hiint(v[1])), "r"(__double2loint(v[2])), "r"(__double2hiint(v[2])),
-        "r"(__double2loint(v[3])), "r"(__double2hiint(v[3]))
-        : "memory");
+// 4 rows' alpha, gamma and delta of every lane to 24 columns of the warp's lanes.
+__device__ __forceinline__ void tmem_store_rows(uint32_t addr, const double (&al)[4],
+                                                const double (&ga)[4], const double (&de)[4]) {
+    __syncwarp();
+    auto put = [](uint32_t at, const double (&v)[4]) {
+        asm volatile(
+            "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(
+                at),
+            "r"(__double2loint(v[0])), "r"(__double2hiint(v[0])), "r"(__double2loint(v[1])),
+            "r"(__double2hiint(v[1])), "r"(__double2loint(v[2])), "r"(__double2hiint(v[2])),
+            "r"(__double2loint(v[3])), "r"(__double2hiint(v[3]))
+            : "memory");
+    };
+    put(addr, al);
+    put(addr + 8, ga);
+    put(addr + 16, de);
 }
-// The registers are valid after tmem_wait_ld on them.
-__device__ __forceinline__ void tmem_load4(uint32_t addr, uint32_t (&w)[8]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]),
-          "=r"(w[7])
-        : "r"(addr)
-        : "memory");
-}
-// Waits for the warp's loads; the registers pass through, so that no use of
-// them moves above it.
-__device__ __forceinline__ void tmem_wait_ld(uint32_t (&u)[8], uint32_t (&v)[8],
-                                             uint32_t (&w)[8]) {
+// The 24 columns back into registers; the wait passes them through, so that no use
+// of them moves above it.
+__device__ __forceinline__ void tmem_load_rows(uint32_t addr, uint32_t (&u)[8], uint32_t (&v)[8],
+                                               uint32_t (&w)[8]) {
+    __syncwarp();
+    auto get = [](uint32_t at, uint32_t (&r)[8]) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+              "=r"(r[7])
+            : "r"(at)
+            : "memory");
+    };
+    get(addr, u);
+    get(addr + 8, v);
+    get(addr + 16, w);
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(u[0]), "+r"(u[1]), "+r"(u[2]), "+r"(u[3]), "+r"(u[4]), "+r"(u[5]),
                    "+r"(u[6]), "+r"(u[7]), "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]),
@@ -458,10 +475,7 @@ tile_wide_kernel(const __grid_constant__ std::conditional_t<GEN, WideMapsGen, Wi
                 }
                 const int kn = (j + 1) * RPS;
                 if (kn <= TR && kn % 4 == 0) {
-                    __syncwarp();
-                    tmem_store4(tcol + (kn - 4) * 6, ta);
-                    tmem_store4(tcol + (kn - 4) * 6 + 8, tg);
-                    tmem_store4(tcol + (kn - 4) * 6 + 16, td);
+                    tmem_store_rows(tcol + (kn - 4) * 6, ta, tg, td);
                 }
             }
             if constexpr (PAD) f.ab0 = r0 == 0 ? 0.0 : f.ab0;  // no row above the first
@@ -572,15 +586,11 @@ tile_wide_kernel(const __grid_constant__ std::conditional_t<GEN, WideMapsGen, Wi
             xn = de[k - TR] - al[k - TR] * x_first - ga[k - TR] * xn;
             put(k, xn);
         }
-        __syncwarp();
         tmem_wait_st();
 #pragma unroll
         for (int k0 = TR - 4; k0 >= 0; k0 -= 4) {
             uint32_t wa[8], wg[8], wd[8];
-            tmem_load4(tcol + k0 * 6, wa);
-            tmem_load4(tcol + k0 * 6 + 8, wg);
-            tmem_load4(tcol + k0 * 6 + 16, wd);
-            tmem_wait_ld(wa, wg, wd);
+            tmem_load_rows(tcol + k0 * 6, wa, wg, wd);
 #pragma unroll
             for (int r = 3; r >= 0; --r) {
                 if (k0 + r == 0) continue;  // row 0 is x_first
