@@ -11,39 +11,9 @@ struct AnyPlan {
 
 template <bool ASYNC, bool CLUSTER>
 int launch_any(const AnyMaps& maps, const AnyArgs& a, cudaStream_t st) {
-    auto kern = tile_any_kernel<ASYNC, CLUSTER>;
-    static bool attr_done = false;
-    if (!attr_done) {
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                max_smem_optin()));
-        attr_done = true;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(any_threads(a.sys, a.nsc), 1, 1);
-    cfg.dynamicSmemBytes = any_smem_bytes(a.sys, a.nsc, a.cl, a.nst, 8);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = a.cl;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = CLUSTER ? 1 : 0;
-    int n = 0;
-    if (CLUSTER) {
-        cfg.gridDim = dim3(a.cl * num_sms(), 1, 1);
-        CK(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
-        if (n <= 0) return fail(BTDMA_ERR_UNSUPPORTED, "no cluster of %d CTAs fits", a.cl);
-    } else {
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, (int)cfg.blockDim.x,
-                                                         cfg.dynamicSmemBytes));
-        // tensor memory is shared by the CTAs of an SM
-        n = std::min(n, 512 / wide_tmem_cols((int)cfg.blockDim.x / 32));
-        n = num_sms() * std::max(1, n);
-    }
-    cfg.gridDim = dim3(std::min(n, a.n_groups) * a.cl, 1, 1);
-    CK(cudaLaunchKernelEx(&cfg, kern, maps, a));
-    return BTDMA_OK;
+    return launch_tmem<tile_any_kernel<ASYNC, CLUSTER>, CLUSTER>(
+        any_threads(a.sys, a.nsc), any_smem_bytes(a.sys, a.nsc, a.cl, a.nst, 8), a.cl,
+        a.n_groups, st, maps, a);
 }
 
 // The fewest CTAs a system, then the fewest sub-segments, of at most 32 rows (one

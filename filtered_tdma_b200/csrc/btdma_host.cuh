@@ -418,25 +418,53 @@ inline TilePlan tile_wide_plan(int n_row, int n_sys, bool cyclic, int elem, bool
     return pl;
 }
 
-template <int SYS, bool CYCLIC, typename TIN, bool FILT = false>
-int launch_tile_wide(const CUtensorMap* maps, const TileArgs& a, cudaStream_t st) {
-    auto kern = tile_wide_kernel<SYS, CYCLIC, TIN, FILT>;
-    WideMaps wm;
-    std::copy(maps, maps + 4, wm.full);
+// Launch of a persistent kernel whose CTAs hold tensor memory, cl of them (a cluster when
+// CLUSTER) per group: as many as are resident at once, or as there are groups.
+template <auto KERN, bool CLUSTER, typename... Args>
+int launch_tmem(int threads, size_t smem, int cl, int n_groups, cudaStream_t st,
+                const Args&... args) {
     static bool attr_done = false;
     if (!attr_done) {
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        CK(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 max_smem_optin()));
         attr_done = true;
     }
-    const int threads = SYS * a.nseg;
-    const size_t smem = tile_wide_smem_bytes(SYS, a.nseg, a.nst, (int)sizeof(TIN));
-    int nb = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, threads, smem));
-    const int grid = std::min(num_sms() * std::max(1, nb), a.n_groups);
-    kern<<<grid, threads, smem, st>>>(wm, a, WideGen{});
-    CK(cudaGetLastError());
+    const int cols = wide_tmem_cols(threads / 32);
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes =
+        CLUSTER ? wide_cluster_smem(smem, cols, (size_t)max_smem_per_sm()) : smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cl;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = CLUSTER ? 1 : 0;
+    int n = 0;
+    if (CLUSTER) {
+        cfg.gridDim = dim3(cl * num_sms(), 1, 1);
+        CK(cudaOccupancyMaxActiveClusters(&n, KERN, &cfg));
+        if (n <= 0) return fail(BTDMA_ERR_UNSUPPORTED, "no cluster of %d CTAs fits", cl);
+    } else {
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, KERN, threads,
+                                                         cfg.dynamicSmemBytes));
+        n = std::min(n, 512 / cols);  // the CTAs of an SM share its columns
+        n = num_sms() * std::max(1, n);
+    }
+    cfg.gridDim = dim3(std::min(n, n_groups) * cl, 1, 1);
+    CK(cudaLaunchKernelEx(&cfg, KERN, args...));
     return BTDMA_OK;
+}
+
+template <int SYS, bool CYCLIC, typename TIN, bool FILT = false>
+int launch_tile_wide(const CUtensorMap* maps, const TileArgs& a, cudaStream_t st) {
+    WideMaps wm;
+    std::copy(maps, maps + 4, wm.full);
+    return launch_tmem<tile_wide_kernel<SYS, CYCLIC, TIN, FILT>, false>(
+        SYS * a.nseg, tile_wide_smem_bytes(SYS, a.nseg, a.nst, (int)sizeof(TIN)), 1, a.n_groups,
+        st, wm, a, WideGen{});
 }
 
 template <typename TIN, bool FILT = false>

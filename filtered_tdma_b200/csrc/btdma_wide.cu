@@ -10,40 +10,10 @@ struct WidePlan {
 
 template <int SYS, bool CYCLIC, typename TIN, bool CLUSTER>
 int launch_wide(const WideMapsGen& maps, const TileArgs& a, const WideGen& gen, cudaStream_t st) {
-    auto kern = tile_wide_kernel<SYS, CYCLIC, TIN, false, true, CLUSTER>;
-    static bool attr_done = false;
-    if (!attr_done) {
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                max_smem_optin()));
-        attr_done = true;
-    }
     const bool odd = sizeof(TIN) == 8 && (a.n_sys & 1) != 0;
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(SYS * a.nseg, 1, 1);
-    cfg.dynamicSmemBytes = tile_wide_smem_bytes(SYS, a.nseg, a.nst, (int)sizeof(TIN), odd, a.cl);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = a.cl;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = CLUSTER ? 1 : 0;
-    int n = 0;
-    if (CLUSTER) {
-        cfg.gridDim = dim3(a.cl * num_sms(), 1, 1);
-        CK(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
-        if (n <= 0) return fail(BTDMA_ERR_UNSUPPORTED, "no cluster of %d CTAs fits", a.cl);
-    } else {
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, (int)cfg.blockDim.x,
-                                                         cfg.dynamicSmemBytes));
-        // tensor memory is shared by the CTAs of an SM
-        n = std::min(n, 512 / wide_tmem_cols((int)cfg.blockDim.x / 32));
-        n = num_sms() * std::max(1, n);
-    }
-    cfg.gridDim = dim3(std::min(n, a.n_groups) * a.cl, 1, 1);
-    CK(cudaLaunchKernelEx(&cfg, kern, maps, a, gen));
-    return BTDMA_OK;
+    return launch_tmem<tile_wide_kernel<SYS, CYCLIC, TIN, false, true, CLUSTER>, CLUSTER>(
+        SYS * a.nseg, tile_wide_smem_bytes(SYS, a.nseg, a.nst, (int)sizeof(TIN), odd, a.cl),
+        a.cl, a.n_groups, st, maps, a, gen);
 }
 
 template <bool CYCLIC, typename TIN>

@@ -107,6 +107,19 @@ __host__ __device__ __forceinline__ int wide_tmem_cols(int warps) {
     while (c < (warps + 3) / 4 * WIDE_TCOLS) c <<= 1;
     return c;
 }
+// Shared memory a CTA of a cluster asks for when it needs `smem` bytes and `cols` columns:
+// at least half the SM's (sm_bytes, of which every resident CTA takes 1 KB more than it
+// asks for), and more than half with more than 256 columns.  So such a CTA has no other
+// cluster's CTA, of any launch, beside it, and others at most one, whose columns (powers
+// of two) fit wherever they lie.  Without it two clusters, of two launches on two streams,
+// could each have a CTA in tmem_alloc, which waits without a limit, for the columns of a
+// CTA that waits at its cluster's barrier for the other one's peer.  (CTAs without a
+// cluster wait for nobody once they have their columns: they only delay.)
+__host__ __device__ __forceinline__ size_t wide_cluster_smem(size_t smem, int cols,
+                                                             size_t sm_bytes) {
+    const size_t least = sm_bytes / 2 - 1024 + (cols > 256 ? 128 : 0);
+    return smem > least ? smem : least;
+}
 // tcgen05's .sync.aligned instructions need every lane of the warp at the same
 // instruction, and callers come from per-lane branches (stores of systems past the
 // batch, rows past a tail): each of these wrappers converges the warp itself.
