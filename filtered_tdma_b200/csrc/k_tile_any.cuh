@@ -203,15 +203,14 @@ tile_any_kernel(const __grid_constant__ AnyMaps maps, const __grid_constant__ An
             tma_load_3d(dst, mp, (cid + it * ncid) * S, k0, tl ? 0 : c * nsc, &full[islot]);
         }
     };
-    // cp.async form, every thread for its own rows: the next stage to request
-    // (group ig, row ik of the sub-segment) and its slot
-    int ig = 0, ik = 0, islot = 0;
-    auto request = [&]() {
+    // cp.async form, every thread for its own rows: the next stage to request (group ig,
+    // row ik of the sub-segment) into its column at dst
+    int ig = 0, ik = 0;
+    auto request = [&](TIN* dst) {
         if (ig < n_my) {
             const int isys = (cid + ig * ncid) * S + s;
             if (on && isys < args.n_sys) {
                 const size_t o = (size_t)(r0 + ik) * ns + isys;
-                TIN* dst = ring + (size_t)islot * sstride + tid;
 #pragma unroll
                 for (int r = 0; r < RPS; ++r) {
                     if (ik + r < mlen) {
@@ -226,20 +225,24 @@ tile_any_kernel(const __grid_constant__ AnyMaps maps, const __grid_constant__ An
                 ik = 0;
                 ++ig;
             }
-            if (++islot == nst) islot = 0;
         }
         cp_async_commit();
     };
     bool ok = true;
     if constexpr (ASYNC) {
-        for (int t = 0; t < ANY_ASYNC_NST - 1; ++t) request();
+        for (int t = 0; t < ANY_ASYNC_NST - 1; ++t) request(ring + (size_t)t * sstride + tid);
     } else if (warp == 0) {
         for (int t = 0; t < nst && t < total; ++t) issue(t, t);
     }
 
     const int toff = ASYNC ? tid : q * RPS * S + s;
     const int rstep = ASYNC ? cols : S;  // between the rows of a stage
-    const TIN* st = ring + toff;
+    TIN* st = ring + toff;
+    // cp.async form: this thread's column of the slot read one stage ago.  The values
+    // read there are taken into the address, so that the copies into it are issued
+    // after those loads have completed (see loads_done; a thread's own loads suffice,
+    // nobody else reads its column).
+    TIN* pst = st + (size_t)(nst - 1) * sstride;
     int slot = 0;
     uint32_t phase = 0;
     int t = 0;
@@ -258,7 +261,8 @@ tile_any_kernel(const __grid_constant__ AnyMaps maps, const __grid_constant__ An
             bits ^= word_of(a2[r]) ^ word_of(b2[r]) ^ word_of(c2[r]) ^ word_of(d2[r]);
         }
         if constexpr (ASYNC) {
-            request();  // into the slot read one stage ago
+            request(pst);
+            pst = st + (bits & zero);
         } else {
             const unsigned z = loads_done(bits, zero);
             if (lane == 0) mbar_arrive(&empty[slot] + z);

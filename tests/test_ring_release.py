@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("n_sys,n_row,P,cyclic,f32", [
     (65536, 512, 8, False, False), (65536, 512, 8, False, True), (20000, 250, 4, False, False),
     (22585, 512, 8, False, False), (4096, 2048, 16, False, False), (40000, 192, 4, True, False),
-    (2048, 128, 4, False, False)])
+    (2048, 128, 4, False, False),
+    (40001, 85, 4, True, False), (4589, 1537, 16, True, False)])  # cp.async rings
 def test_repeated_solves_bit_identical(cuda, n_sys, n_row, P, cyclic, f32):
     import torch
     dt = torch.float32 if f32 else torch.float64
@@ -31,3 +32,38 @@ def test_repeated_solves_bit_identical(cuda, n_sys, n_row, P, cyclic, f32):
             first = X.clone()
         assert torch.equal(X, first)
     assert s.status() == 0
+
+
+@pytest.mark.parametrize("app", ["heat", "momentum", "poisson"])
+def test_repeated_application_steps_bit_identical(cuda, app):
+    import torch
+
+    from filtered_tdma_b200.heat import HeatADI
+    from filtered_tdma_b200.momentum import ChannelMomentum
+    from filtered_tdma_b200.poisson import ChannelPoisson
+    g = torch.Generator(device=cuda).manual_seed(11)
+    if app == "poisson":
+        p = ChannelPoisson(128, 64, 96)
+        start = torch.view_as_complex(torch.rand((96, p.n_modes, 2), generator=g, device=cuda,
+                                                 dtype=torch.float64))
+    else:
+        start = torch.rand((66, 130, 98), generator=g, device=cuda, dtype=torch.float64)
+    h = HeatADI(96, 128, 64, dt=3e-4) if app == "heat" else None
+    m = ChannelMomentum(96, 128, 64, pbc_x=False) if app == "momentum" else None
+    flush = torch.empty(1 << 25, dtype=torch.float64, device=cuda)
+    first = None
+    for i in range(40):
+        if i % 4 == 0:
+            flush.fill_(i)
+        x = start.clone()
+        if app == "heat":
+            h.step(x, 2, graph=False)
+        elif app == "momentum":
+            q = torch.zeros_like(x)
+            m.adi(1, x, q, 1e-3)
+            x = q
+        else:
+            p.solve(x)
+        if first is None:
+            first = x
+        assert torch.equal(x, first)
