@@ -128,6 +128,7 @@ int tile_wide_gen(const TIN* A, const TIN* B, const TIN* C, const TIN* D, double
         gen.nl = p.nsc;
     }
     for (int f = 0; f < 4; ++f) {
+        if constexpr (sizeof(TIN) == 8) gen.in[f] = src[f];
         if ((cyclic || p.cl > 1) &&
             !wide_map(&maps.full[f], src[f], n_sys, WIDE_M, nfull, p.sys, p.nsc, elem, odd))
             return 0;

@@ -79,6 +79,7 @@ struct WideGen {
     int tail;   // rows of the tail sub-segment (0: periodic, none)
     int nl;     // sub-segments before it in the last CTA
     int empty;  // bit f: array f has no (pair of) rows in the tail's box
+    const double* in[4];  // A, B, C, D (FP64), for passes with PIV_EXACT
 };
 
 // Elements of a ring stage; odd n_sys: a box per array and row of NSC pieces of
@@ -229,17 +230,46 @@ struct WideFwd {
     double gm2;            // gamma of row M-2
 };
 
+// The reciprocals of a forward pass.  rcp_nr wants normal pivots with normal reciprocals.
+// The form that also serves row counts and batches outside the narrow kernel's keeps the
+// whole FP64 range all the same: PIV_WATCH notes pivots of 2^1017 and more (one above
+// 2^1022 would pass with a reciprocal of 0), subnormal and infinite ones leave NaN, and a
+// warp with such a system takes its rows again from global memory with PIV_EXACT, where
+// that system's lanes use correctly rounded reciprocals.  (B200, 62500 x 250: 110 us
+// unwatched, 113 watched; correctly rounded ones throughout, or a check and a branch a
+// row, 114, and 4 to 7 % over clusters, where the watch costs nothing.)
+enum Pivots { PIV_NORMAL = 0, PIV_WATCH = 1, PIV_EXACT = 2 };
+struct PivotWatch {
+    float big = 0.0f;    // PIV_WATCH: NaN once a pivot's high word was, read as a float
+    bool exact = false;  // PIV_EXACT: this lane's system needs it
+};
+template <int PIV>
+__device__ __forceinline__ double wide_rcp(double x, PivotWatch& pw) {
+    if constexpr (PIV == PIV_WATCH)
+        pw.big = fmaf(__int_as_float(__double2hiint(x)), 0.0f, pw.big);
+    double r = rcp_nr(x);
+    if constexpr (PIV == PIV_EXACT) {
+        if (pw.exact) r = Exact64::rcp(x);
+    }
+    return r;
+}
+// Whether a sub-segment's pass met a pivot outside rcp_nr's range (or NaN in the data); d0
+// and dep: the right-hand sides of its row 0, whose chain ends there, and its last row.
+__device__ __forceinline__ bool pivots_out_of_range(const PivotWatch& pw, double d0, double dep) {
+    return isnan(pw.big) || isnan(d0) || isnan(dep);
+}
 // Row k of the forward pass (the expressions of k_tile.cuh's loop, FP64).
+template <int PIV>
 __device__ __forceinline__ void wide_row(WideFwd& f, int k, double a, double b, double cc,
-                                         double d) {
+                                         double d, PivotWatch& pw) {
     constexpr int M = WIDE_M;
     if (k == 0) {
-        const double ib = rcp_nr(b);
+        const double ib = wide_rcp<PIV>(b, pw);
         f.ab0 = a * ib;
         f.cb0 = cc * ib;
         f.db0 = d * ib;
     } else if (k == 1) {
-        const double ib = rcp_nr(b);
+        const double ib = wide_rcp<PIV>(b, pw);
         f.alp = a * ib;
         f.gap = cc * ib;
         f.dep = d * ib;
@@ -247,7 +277,7 @@ __device__ __forceinline__ void wide_row(WideFwd& f, int k, double a, double b, 
         f.sa = f.alp;
         f.sd = f.dep;
     } else {
-        const double inv = rcp_nr(b - a * f.gap);
+        const double inv = wide_rcp<PIV>(b - a * f.gap, pw);
         const double g = cc * inv;
         const double e = (d - a * f.dep) * inv;
         const double l = -a * f.alp * inv;
@@ -290,6 +320,7 @@ tile_wide_kernel(const __grid_constant__ std::conditional_t<GEN, WideMapsGen, Wi
     constexpr int SPG = M / RPS;  // stages per group
     constexpr int RP = SYS + 1;
     constexpr bool PAD = GEN && !CYCLIC;
+    constexpr int PIV = GEN && sizeof(TIN) == 8 ? PIV_WATCH : PIV_NORMAL;
     // a closed gate: nothing to do (TILE_MODE_GATE_ZERO: open while *gate == 0); every
     // CTA reads the same word
     if (!GEN && args.gate != nullptr &&
@@ -466,6 +497,7 @@ tile_wide_kernel(const __grid_constant__ std::conditional_t<GEN, WideMapsGen, Wi
         double al[M - TR], ga[M - TR], de[M - TR];  // rows TR .. M - 1
         {
             WideFwd f = {};
+            PivotWatch pw;
             double ta[4], tg[4], td[4];  // rows of the 4-row block going to tensor memory
 #pragma unroll
             for (int j = 0; j < SPG; ++j) {
@@ -475,7 +507,7 @@ tile_wide_kernel(const __grid_constant__ std::conditional_t<GEN, WideMapsGen, Wi
                 for (int r = 0; r < RPS; ++r) {
                     const int k = j * RPS + r;
                     if constexpr (PAD) b2[r] = k < mlen ? b2[r] : 1.0;
-                    wide_row(f, k, a2[r], b2[r], c2[r], d2[r]);
+                    wide_row<PIV>(f, k, a2[r], b2[r], c2[r], d2[r], pw);
                     if (k < TR) {
                         ta[k % 4] = f.alp;
                         tg[k % 4] = f.gap;
@@ -489,6 +521,49 @@ tile_wide_kernel(const __grid_constant__ std::conditional_t<GEN, WideMapsGen, Wi
                 const int kn = (j + 1) * RPS;
                 if (kn <= TR && kn % 4 == 0) {
                     tmem_store_rows(tcol + (kn - 4) * 6, ta, tg, td);
+                }
+            }
+            if constexpr (PIV == PIV_WATCH) {
+                pw.exact = valid && pivots_out_of_range(pw, f.db0, f.dep);
+                if (__builtin_expect(__any_sync(0xffffffffu, pw.exact), 0)) {
+                    f = {};
+                    // rows k .. k + 3 of the pass; a row past the system's end is an
+                    // identity row, and its last row has no coupling below (PAD)
+                    auto rows4 = [&](int k, bool first, bool last) {
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            double v[4] = {0.0, 1.0, 0.0, 0.0};
+                            if (valid && k + r < mlen) {
+                                const size_t o = (size_t)(r0 + k + r) * ns + sys;
+#pragma unroll
+                                for (int i = 0; i < 4; ++i)
+                                    if (!PAD || i != 2 || r0 + k + r + 1 < args.n_row)
+                                        v[i] = gen.in[i][o];
+                            }
+                            wide_row<PIV_EXACT>(f, first ? r : (last ? M - 4 + r : 4), v[0], v[1],
+                                                v[2], v[3], pw);
+                            ta[r] = f.alp;
+                            tg[r] = f.gap;
+                            td[r] = f.dep;
+                        }
+                    };
+                    rows4(0, true, false);
+                    tmem_store_rows(tcol, ta, tg, td);
+#pragma unroll 1
+                    for (int k = 4; k < TR; k += 4) {
+                        rows4(k, false, false);
+                        tmem_store_rows(tcol + k * 6, ta, tg, td);
+                    }
+#pragma unroll
+                    for (int k = TR; k < M; k += 4) {
+                        rows4(k, false, k == M - 4);
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            al[k - TR + r] = ta[r];
+                            ga[k - TR + r] = tg[r];
+                            de[k - TR + r] = td[r];
+                        }
+                    }
                 }
             }
             if constexpr (PAD) f.ab0 = r0 == 0 ? 0.0 : f.ab0;  // no row above the first

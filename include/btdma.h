@@ -89,11 +89,13 @@ enum btdma_flags {
      * bit-identical to PaScaLTDMA::solve with nprocs = P
      * (libs/pascal_tdma/cpu/pascal_tdma.cpp:113-227).  Without the flag PaScaL
      * uses the register-tiled kernel, exact to rounding (<= 1e-12 relative to
-     * the serial Thomas) and faster.  For Filtered handles the flag runs the
-     * reference's scheme in its operation order (segment kernels, J-row
-     * cut-off) and keeps its 2x2 interface where J >= m - 2 (no exact
-     * fallback), so every Filtered result is bit-identical to the
-     * reference's. */
+     * the serial Thomas) and faster.  (Where 16 divides n_row and n_sys is even,
+     * its pivots and their reciprocals must be normal numbers; elsewhere, as with
+     * the flag, subnormal, largest and infinite pivots are served too.)  For
+     * Filtered handles the flag runs the reference's scheme in its operation
+     * order (segment kernels, J-row cut-off) and keeps its 2x2 interface where
+     * J >= m - 2 (no exact fallback), so every Filtered result is
+     * bit-identical to the reference's. */
     BTDMA_FLAG_REFERENCE_ORDER = 1 << 1
 };
 
