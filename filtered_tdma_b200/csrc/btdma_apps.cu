@@ -97,15 +97,16 @@ int heat_enqueue(btdma_heat_t h, double* theta, cudaStream_t st, cudaEvent_t* ev
     rc = shared(SH_HEAT, 0, theta, h->buf1, g.ix * g.iy, g.iz, g.ix, g.iz * g.ix, 1, g.ix, 0.0, 1,
                 h->cosx, h->cosy);
     if (rc < 0) return rc;
-    if (rc == 0) {
-        if (g.iz <= 32 * TILE_MT)
-            return fail(BTDMA_ERR_UNSUPPORTED, "Z sweep: theta must be 16-byte aligned");
+    if (rc == 0) {  // a longer axis, or theta off 16 bytes: the right-hand side as a pass
         heat_rhs_z_kernel<<<dim3((g.ix + 127) / 128, g.iy, (g.iz + HEAT_KCH - 1) / HEAT_KCH), b1,
                             0, st>>>(theta, h->buf0, g);
         CK(cudaGetLastError());
         mark(1);
-        if ((rc = sweep(0, h->buf0, h->buf1, g.ix * g.iy, g.iz, g.bz, g.ix, g.iz * g.ix, 1, g.ix,
-                        "Z")))
+        rc = shared(SH_ROWS, 0, h->buf0, h->buf1, g.ix * g.iy, g.iz, g.ix, g.iz * g.ix, 1, g.ix,
+                    0.0, 1, nullptr, nullptr);
+        if (rc < 0) return rc;
+        if (rc == 0 && (rc = sweep(0, h->buf0, h->buf1, g.ix * g.iy, g.iz, g.bz, g.ix,
+                                   g.iz * g.ix, 1, g.ix, "Z")))
             return rc;
     }
     mark(2);
