@@ -22,7 +22,6 @@ struct btdma_heat {
     double* buf1 = nullptr;  // Y sweep layout
     double* err = nullptr;   // L2 accumulator
     double* hpar = nullptr;  // {bx, by, dt 3 pi^2, iy, iz} for the fused Z sweep
-    double* scratch = nullptr;  // full grid, the warm-up step before graph capture
     double* tab = nullptr;      // factor tables of the Z, Y, X sweeps, tab_stride apart
     size_t tab_stride = 0;      // (built once at create: the matrices are fixed)
     unsigned* status = nullptr;
@@ -205,7 +204,6 @@ int btdma_heat_create(int ix, int iy, int iz, double dt, btdma_heat_t* out) {
     CKH(cudaMalloc(&h->buf0, sizeof(double) * inner));
     CKH(cudaMalloc(&h->buf1, sizeof(double) * inner));
     CKH(cudaMalloc(&h->err, sizeof(double)));
-    CKH(cudaMalloc(&h->scratch, sizeof(double) * (size_t)(ix + 2) * (iy + 2) * (iz + 2)));
     h->tab_stride = gen_table_doubles(std::max(ix, std::max(iy, iz)));
     CKH(cudaMalloc(&h->tab, sizeof(double) * 3 * h->tab_stride));
     CKH(cudaMalloc(&h->status, sizeof(unsigned)));
@@ -260,7 +258,6 @@ int btdma_heat_destroy(btdma_heat_t h) {
     cudaFree(h->buf1);
     cudaFree(h->err);
     cudaFree(h->hpar);
-    cudaFree(h->scratch);
     cudaFree(h->tab);
     cudaFree(h->status);
     delete h;
@@ -294,22 +291,12 @@ int btdma_heat_step(btdma_heat_t h, double* theta, int n_steps, int use_graph,
         if (h->graph) cudaGraphDestroy(h->graph);
         h->exec = nullptr;
         h->graph = nullptr;
-        // one uncaptured step on a zeroed scratch field first, so the kernels'
-        // first-use attribute calls stay out of the capture (theta is untouched);
-        // after the caller's earlier steps, which may still use the sweep buffers
-        const HeatGeom& g = h->g;
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        CK(cudaStreamIsCapturing(stream, &cap));
-        if (cap == cudaStreamCaptureStatusNone) CK(cudaStreamSynchronize(stream));
-        CK(cudaMemsetAsync(h->scratch, 0, sizeof(double) * (size_t)(g.ix + 2) * (g.iy + 2) *
-                                              (g.iz + 2), h->cap));
-        int rc = heat_enqueue(h, h->scratch, h->cap);
-        if (rc) return rc;
-        CK(cudaStreamSynchronize(h->cap));
-        // capture on the private stream, after the caller's stream has reached
-        // this point (the graph is launched on the caller's stream below)
+        // captured on the private stream, where nothing runs, and launched on the
+        // caller's below: no step in flight shares its buffers with the capture, and the
+        // host waits for nothing (the kernels' first-use attribute calls are no stream
+        // work and may come in a capture)
         CK(cudaStreamBeginCapture(h->cap, cudaStreamCaptureModeThreadLocal));
-        rc = heat_enqueue(h, theta, h->cap);
+        const int rc = heat_enqueue(h, theta, h->cap);
         cudaGraph_t gr = nullptr;
         const cudaError_t e = cudaStreamEndCapture(h->cap, &gr);
         if (rc) {
