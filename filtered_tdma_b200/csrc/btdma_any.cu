@@ -60,9 +60,9 @@ AnyPlan any_plan(int n_row, int n_sys, bool tma) {
 }  // namespace
 
 int tile_any_solve(const double* A, const double* B, const double* C, const double* D, double* X,
-                   int n_sys, int n_row, unsigned* status, cudaStream_t st) {
+                   int n_sys, int n_row, unsigned* status, cudaStream_t st, int n_plan) {
     const double* src[4] = {A, B, C, D};
-    bool tma = true;
+    bool tma = n_plan % 2 == 0;
     for (const double* p : src) tma = tma && tma_ok(p, n_sys);
     const AnyPlan p = any_plan(n_row, n_sys, tma);
     if (p.sys == 0) return 0;

@@ -93,8 +93,8 @@ bool seg_fits(btdma_t h, int n_sys, int n_row, bool cyclic) {
            (n_sys + SEG_S - 1) / SEG_S <= 65535;
 }
 
-// n_plan: systems of the whole batch this call solves a part of (btdma_solve_host's
-// chunks run the kernels the whole batch would).
+// n_plan: systems of the whole batch this call solves a part of: btdma_solve_host's
+// chunks cut a system as the whole batch would, an odd batch's even chunks too.
 int solve_impl(btdma_t h, const double* A, const double* B, const double* C, const double* D,
                double* X, int n_sys, int n_row, bool cyclic, cudaStream_t st, int n_plan) {
     int rc = check_sizes(h, n_sys, n_row);
@@ -154,14 +154,14 @@ int solve_impl(btdma_t h, const double* A, const double* B, const double* C, con
         // segments, whose shorter sweeps are faster there (B200, P = 4: 512 x 50
         // 9.5 us against 10.2, 2048 x 50 9.8 / 10.3, 8192 x 50 10.8 / 10.4).
         const bool general = seg_fits(h, n_sys, n_row, cyclic) &&
-                             !(n_sys % 2 == 0 && n_plan <= 4096 &&
+                             !(n_plan % 2 == 0 && n_plan <= 4096 &&
                                (n_row + h->P - 1) / h->P <= 16);
         rc = try_tile<double>(A, B, C, D, X, n_sys, n_row, cyclic, h->status, st, false,
                               nullptr, h->tile_shape, 0, false, general, n_plan);
         if (rc < 0) return rc;
         if (rc == 1) return BTDMA_OK;
         if (general && cyclic && h->tile_shape == BTDMA_TILE_AUTO) {
-            rc = tile_any_solve(A, B, C, D, X, n_sys, n_row, h->status, st);
+            rc = tile_any_solve(A, B, C, D, X, n_sys, n_row, h->status, st, n_plan);
             if (rc < 0) return rc;
             if (rc == 1) return BTDMA_OK;
         }

@@ -39,9 +39,10 @@ int tile_wide_gen(const TIN* A, const TIN* B, const TIN* C, const TIN* D, double
                   int n_row, bool cyclic, unsigned* status, cudaStream_t st, bool narrow,
                   int n_plan);
 // Periodic FP64 systems whose row count is not 32 x a power of two
-// (btdma_any.cu).  Returns as tile_solve_batch.
+// (btdma_any.cu); an odd n_plan takes the forms for an odd n_sys.  Returns as
+// tile_solve_batch.
 int tile_any_solve(const double* A, const double* B, const double* C, const double* D, double* X,
-                   int n_sys, int n_row, unsigned* status, cudaStream_t st);
+                   int n_sys, int n_row, unsigned* status, cudaStream_t st, int n_plan);
 
 // A shared-matrix sweep (btdma_sh.cu): `a` without its plan fields; src is D
 // [n_row][n_sys] (SH_ROWS) or the ghosted field of nx x ny cells a plane.  Returns as
@@ -495,8 +496,8 @@ inline bool tma_ok_elem(const void* p, int n_sys, int elem) {
 // 0: Filtered's reduced system with segments of filt_r sub-segments.
 // shape: BTDMA_TILE_* (the wide kernel serves FP64-arithmetic solves that do not
 // accumulate; its general form serves AUTO's exact ungated ones, and with
-// `general` also shapes the narrow kernel does not take).  n_plan: the batch size
-// AUTO chooses for (0: n_sys).
+// `general` also shapes the narrow kernel does not take).  n_plan: the batch size,
+// odd or even, that AUTO chooses for (0: n_sys).
 template <typename TIN, typename TC = double>
 int try_tile(const TIN* A, const TIN* B, const TIN* C, const TIN* D, double* X, int n_sys,
              int n_row, bool cyclic, unsigned* status, cudaStream_t st, bool accumulate = false,
@@ -505,7 +506,8 @@ int try_tile(const TIN* A, const TIN* B, const TIN* C, const TIN* D, double* X, 
     const int elem = (int)sizeof(TIN);
     if (n_plan <= 0) n_plan = n_sys;
     const bool aligned = tma_ok_elem(A, n_sys, elem) && tma_ok_elem(B, n_sys, elem) &&
-                         tma_ok_elem(C, n_sys, elem) && tma_ok_elem(D, n_sys, elem);
+                         tma_ok_elem(C, n_sys, elem) && tma_ok_elem(D, n_sys, elem) &&
+                         tma_ok_elem(A, n_plan, elem);
     bool wide = false;
     TilePlan pl;
     if (shape != BTDMA_TILE_NARROW && sizeof(TC) == 8 && !accumulate && aligned) {
