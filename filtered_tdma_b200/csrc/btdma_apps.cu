@@ -21,7 +21,6 @@ struct btdma_heat {
     double* buf0 = nullptr;  // Z and X sweep layouts
     double* buf1 = nullptr;  // Y sweep layout
     double* err = nullptr;   // L2 accumulator
-    double* hpar = nullptr;  // {bx, by, dt 3 pi^2, iy, iz} for the fused Z sweep
     double* tab = nullptr;      // factor tables of the Z, Y, X sweeps, tab_stride apart
     size_t tab_stride = 0;      // (built once at create: the matrices are fixed)
     unsigned* status = nullptr;
@@ -37,9 +36,8 @@ namespace {
 // One step as a kernel sequence on stream st (no host sync): the Z, Y and X sweeps,
 // each storing its solution in the layout of the next one (X: into theta), with the
 // right-hand side formed in the Z sweep and the Y and X wall terms in theirs.  Grids
-// with an axis longer than the shared-matrix sweeps take (512 rows) run the older
-// kernels for it: the right-hand side, wall folds and transposes as passes of their
-// own.  ev (optional): 8 events recorded around the phases (the profiled step).
+// with an axis longer than the shared-matrix sweeps take (512 rows) run the general
+// kernels for it: the right-hand side and the wall folds as passes of their own.  ev (optional): 8 events recorded around the phases (the profiled step).
 int heat_enqueue(btdma_heat_t h, double* theta, cudaStream_t st, cudaEvent_t* ev = nullptr) {
     const HeatGeom& g = h->g;
     auto mark = [&](int i) {
@@ -195,11 +193,6 @@ int btdma_heat_create(int ix, int iy, int iz, double dt, btdma_heat_t* out) {
     CKH(upload(&h->cosx, kx));
     CKH(upload(&h->cosy, ky));
     CKH(upload(&h->cosz, kz));
-    {
-        const double bx = dt / (2.0 * (2.0 / ix) * (2.0 / ix));
-        const double by = dt / (2.0 * (2.0 / iy) * (2.0 / iy));
-        CKH(upload(&h->hpar, {bx, by, dt * 3.0 * HEAT_PI * HEAT_PI, (double)iy, (double)iz}));
-    }
     const size_t inner = (size_t)ix * iy * iz;
     CKH(cudaMalloc(&h->buf0, sizeof(double) * inner));
     CKH(cudaMalloc(&h->buf1, sizeof(double) * inner));
@@ -257,7 +250,6 @@ int btdma_heat_destroy(btdma_heat_t h) {
     cudaFree(h->buf0);
     cudaFree(h->buf1);
     cudaFree(h->err);
-    cudaFree(h->hpar);
     cudaFree(h->tab);
     cudaFree(h->status);
     delete h;

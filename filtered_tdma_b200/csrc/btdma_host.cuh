@@ -584,9 +584,9 @@ int build_gen_table(int n_row, const TileArgs& gen, double* tab, cudaStream_t st
     return BTDMA_OK;
 }
 
-// Generated-coefficient batch, only D read (the GEN modes of the tiled
-// kernel; GEN 1 and 3 for systems above 32 sub-segments, which k_tile_sh.cuh does not
-// take; the coefficient fields of `gen` are used, the rest is filled here).
+// Generated-coefficient batch, only D read (the GEN modes of the tiled kernel, for
+// systems above 32 sub-segments, which k_tile_sh.cuh and k_poisson.cuh do not take;
+// the coefficient fields of `gen` are used, the rest is filled here).
 // Returns 1 when launched, 0 when the shape is not tiled, < 0 on error.
 // GEN 1 and 3 (one matrix for every system): `tab` is device scratch of
 // gen_table_doubles(n_row) doubles for the shared elimination factors, built
@@ -596,7 +596,8 @@ int try_tile_gen(const double* D, double* X, int n_sys, int n_row, const TileArg
                  unsigned* status, cudaStream_t st, double* tab = nullptr,
                  bool table_ready = false) {
     const TilePlan pl = tile_plan(n_row, CYC, 8, 1, GEN == 1 || GEN == 3);
-    if (pl.sys == 0 || !tma_ok_elem(D, n_sys, 8)) return 0;
+    // above 32 sub-segments: 16 systems a cluster
+    if (pl.sys != 16 || pl.nseg <= 32 || !tma_ok_elem(D, n_sys, 8)) return 0;
     const int nsc = pl.nseg / pl.cl;
     CUtensorMap maps[4];
     if (!make_tile_map(&maps[3], D, n_sys, pl.nseg, pl.sys, nsc, 8, 1)) return 0;
@@ -618,18 +619,7 @@ int try_tile_gen(const double* D, double* X, int n_sys, int n_row, const TileArg
         }
         a.gtab = tab;
     }
-    int rc;
-    if constexpr (GEN == 1 || GEN == 3) {  // above 32 sub-segments: 16 systems a cluster
-        if (pl.sys != 16) return 0;
-        rc = launch_tile_sys<16, CYC, double, double, GEN>(maps, a, st);
-        return rc == BTDMA_OK ? 1 : rc;
-    }
-    switch (pl.sys) {
-        case 128: rc = launch_tile_sys<128, CYC, double, double, GEN>(maps, a, st); break;
-        case 64: rc = launch_tile_sys<64, CYC, double, double, GEN>(maps, a, st); break;
-        case 32: rc = launch_tile_sys<32, CYC, double, double, GEN>(maps, a, st); break;
-        default: rc = launch_tile_sys<16, CYC, double, double, GEN>(maps, a, st); break;
-    }
+    const int rc = launch_tile_sys<16, CYC, double, double, GEN>(maps, a, st);
     return rc == BTDMA_OK ? 1 : rc;
 }
 

@@ -13,7 +13,7 @@ ShPlan sh_plan(const ShArgs& a, int mode, bool cyclic) {
     if (a.n_row % TILE_MT != 0 || a.n_sys % 2 != 0) return p;
     const int nseg = a.n_row / TILE_MT;
     if (nseg > 32 || (cyclic && (nseg & (nseg - 1)) != 0)) return p;
-    int sys = nseg > 16 && mode != SH_HEAT ? 16 : 32;
+    int sys = nseg > 16 && mode != SH_HEAT ? 16 : 32;  // SH_HEAT: always 32
     // SH_FIELD: a group stays in one row of cells; SH_HEAT: whole 16 x sys / 16 blocks
     if (mode == SH_FIELD && a.fblk % sys != 0) sys = 16;
     if (mode == SH_FIELD && a.fblk % sys != 0) return p;
@@ -68,9 +68,11 @@ int launch_sh_store(const CUtensorMap& tm, const ShArgs& a, bool cyclic, int sto
             case SH_ONE * 2 + 1: return launch_sh<SYS, true, MODE, SH_ONE>(tm, a, st);
             default: return launch_sh<SYS, false, MODE, SH_ONE>(tm, a, st);
         }
-    } else {
+    } else if constexpr (MODE == SH_FIELD) {
         return store == SH_PAIR ? launch_sh<SYS, false, MODE, SH_PAIR>(tm, a, st)
                                 : launch_sh<SYS, false, MODE, SH_ONE>(tm, a, st);
+    } else {  // into the library's own buffer
+        return store == SH_PAIR ? launch_sh<SYS, false, MODE, SH_PAIR>(tm, a, st) : 0;
     }
 }
 
@@ -134,6 +136,5 @@ int try_sh(int mode, const double* src, int nx, int ny, ShArgs a, bool cyclic, c
         return launch_sh_store<32, SH_HEAT>(tm, a, cyclic, store, st);
     }
     if (mode == SH_ROWS) return launch_sh_store<16, SH_ROWS>(tm, a, cyclic, store, st);
-    if (mode == SH_FIELD) return launch_sh_store<16, SH_FIELD>(tm, a, cyclic, store, st);
-    return launch_sh_store<16, SH_HEAT>(tm, a, cyclic, store, st);
+    return launch_sh_store<16, SH_FIELD>(tm, a, cyclic, store, st);
 }

@@ -291,7 +291,7 @@ __device__ __forceinline__ void reduced_outer(const double (&f)[3], const double
 
 // The matrix steps of reduced_solve_shfl for one lane, written to lt[0 .. 5 +
 // 3 * levels) (the lane table of a matrix shared by every system, see
-// reduced_solve_rhs).  Every lane of the warp calls it with the same nseg
+// reduced_solve_rhs2).  Every lane of the warp calls it with the same nseg
 // <= 32; lanes with act == false carry identity rows.
 template <bool CYCLIC>
 __device__ __forceinline__ void reduced_lane_table(double l0, double u0, double l1, double u1,
@@ -356,45 +356,11 @@ __device__ __forceinline__ void reduced_lane_table(double l0, double u0, double 
     }
 }
 
-// reduced_solve_shfl for a batch whose systems share one matrix: lt is this
-// lane's table from reduced_lane_table (entry k at lt[k * ls]), so only the
-// right-hand sides travel (two shuffles and three operations per level, no
-// reciprocals).  The right-hand-side arithmetic is that of reduced_solve_shfl.
-template <bool CYCLIC>
-__device__ __forceinline__ void reduced_solve_rhs(double r0, double r1, int p, int nseg, int W,
-                                                  const double* __restrict__ lt, int ls,
-                                                  double& xf, double& xl) {
-    const int pn = (CYCLIC && p == nseg - 1) ? 0 : p + 1;
-    const double r0n = __shfl_sync(0xffffffffu, r0, pn & (W - 1), W);
-    double r = (r1 - lt[1 * ls] * r0 - lt[2 * ls] * r0n) * lt[0 * ls];
-    if (CYCLIC && nseg == 1) {
-        r *= lt[7 * ls];
-    } else {
-#pragma unroll
-        for (int v = 0; v < 5; ++v) {
-            const int dl = 1 << v;
-            if (dl >= nseg) break;
-            int im = p - dl, ip = p + dl;
-            if (CYCLIC) {
-                im = im < 0 ? im + nseg : im;
-                ip = ip >= nseg ? ip - nseg : ip;
-            }
-            const double rm = __shfl_sync(0xffffffffu, r, im & (W - 1), W);
-            const double rp = __shfl_sync(0xffffffffu, r, ip & (W - 1), W);
-            r = (r - lt[(5 + 3 * v) * ls] * rm - lt[(6 + 3 * v) * ls] * rp) * lt[(7 + 3 * v) * ls];
-            if (CYCLIC && 2 * dl == nseg) break;
-        }
-    }
-    xl = r;
-    const int pm = (CYCLIC && p == 0) ? nseg - 1 : p - 1;
-    double xlm = __shfl_sync(0xffffffffu, xl, pm & (W - 1), W);
-    if (!CYCLIC && p == 0) xlm = 0.0;
-    xf = r0 - lt[3 * ls] * xlm - lt[4 * ls] * xl;
-}
-
-// reduced_solve_rhs for two systems a lane (r0, r1 hold the first / last rows' values
-// of both): the table entries are read once, and the two chains fill each other's
-// latency.
+// reduced_solve_shfl for a batch whose systems share one matrix, two systems a lane (r0,
+// r1 hold the first / last rows' values of both): lt is this lane's table from
+// reduced_lane_table (entry k at lt[k * ls]), so only the right-hand sides travel (no
+// reciprocals, arithmetic as in reduced_solve_shfl); the table entries are read once for
+// both, and the two chains fill each other's latency.
 template <bool CYCLIC>
 __device__ __forceinline__ void reduced_solve_rhs2(double2 r0, double2 r1, int p, int nseg, int W,
                                                    const double* __restrict__ lt, int ls,

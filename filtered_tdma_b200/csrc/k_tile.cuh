@@ -114,7 +114,8 @@ struct TileArgs {
             int xblk, xbs, xss, xrs;
         };
     };
-    // Generated-coefficient instantiations read only D:
+    // Generated-coefficient instantiations (more than 32 sub-segments; k_tile_sh.cuh and
+    // k_poisson.cuh take the shorter ones) read only D:
     //  GEN == 1 (heat sweep): every row -cs x_{j-1} + (1 + 2 cs) x_j - cs x_{j+1},
     //    plus cs on the diagonal of the first and last row when cbound != 0
     //    (the fully implicit Dirichlet wall of the heat ADI step);
@@ -131,12 +132,12 @@ struct TileArgs {
     const double* gb;
     const double* gc;
     const double* glam;
-    // GEN 1 and 3 (longer systems than k_tile_sh.cuh takes): every system of the
-    // batch has the same matrix, so the elimination of each sub-segment is computed once (tile_table_kernel) into
+    // GEN 1 and 3: every system of the batch has the same matrix, so the
+    // elimination of each sub-segment is computed once (tile_table_kernel) into
     // gtab: per row [inv pivot, a * inv, pi, alpha, gamma] (n_row x 5), then
     // per sub-segment [r, r c0, l0, u0, l1, u1] (nseg x 6), then (up to 32
-    // sub-segments) the reduced system's lane table at tile_red_offset(n_row);
-    // the solve runs the right-hand-side recurrences only
+    // sub-segments, for k_tile_sh.cuh) the reduced system's lane table at
+    // tile_red_offset(n_row); the solve runs the right-hand-side recurrences only
     const double* gtab;
     int gpin;
     unsigned* status;
@@ -160,17 +161,13 @@ __host__ __device__ __forceinline__ int tile_lanes(int nseg) {
 // Shared memory (doubles unless noted), T = SYS * NSC threads, SUB = SYS / CL,
 // RP = SYS + 1 (padded pitch of the exchange buffers):
 //   ring  NST * NA * RPS * T      TMA stages (A, B, C, D or D only; RPS rows per sub-segment)
-//   red   6 * NSC * RP            this CTA's reduced rows (l0,u0,r0 | l1,u1,r1);
-//                                 2 * NSC * RP (r0 | r1) for a shared matrix of
-//                                 NSEG <= 32, whose l, u come from the lane table
+//   red   6 * NSC * RP            this CTA's reduced rows (l0,u0,r0 | l1,u1,r1)
 //   xr    2 * NSC * RP            x_first / x_last of this CTA's sub-segments
 //   pcr   6 * (NSEG + 2) * SUB    PCR buffers, only when NSEG > 32
 //   tab   tile_tab_doubles(NSC)   shared matrix: this CTA's factor table
-//   lane  32 * TILE_RED_LANE      shared matrix, NSEG <= 32: the lane table
 //   bars  2 * NST mbarriers
-__host__ __device__ __forceinline__ size_t tile_fixed_doubles(int sys, int nsc, int nseg, int sub,
-                                                              bool shared_tab = false) {
-    if (shared_tab && nseg <= 32) return 4ull * nsc * (sys + 1) + 32ull * TILE_RED_LANE;
+__host__ __device__ __forceinline__ size_t tile_fixed_doubles(int sys, int nsc, int nseg,
+                                                              int sub) {
     size_t f = 8ull * nsc * (sys + 1);
     if (nseg > 32) f += 6ull * (nseg + 2) * sub;
     return f;
@@ -195,7 +192,7 @@ __host__ __device__ __forceinline__ size_t tile_smem_bytes(int sys, int nsc, int
                                                            bool shared_tab = false) {
     return tile_ring_bytes(sys, nsc, nst, elem, na) +
            (shared_tab ? tile_tab_doubles(nsc) * sizeof(double) : 0) +
-           tile_fixed_doubles(sys, nsc, nseg, sub, shared_tab) * sizeof(double) +
+           tile_fixed_doubles(sys, nsc, nseg, sub) * sizeof(double) +
            2ull * nst * sizeof(uint64_t) + 128;
 }
 
@@ -265,20 +262,17 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const int sub = SYS / cl;    // systems whose reduced system this CTA solves
     const int W = tile_lanes(nseg);
     const bool shuffled = W <= 32;
-    const bool rhs_red = SH && shuffled;  // reduced matrix from the lane table
     const int fstride = nsc * RP;  // field stride of red / xr
 
     TIN* ring = reinterpret_cast<TIN*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
     const int sstride = tile_stage_elems(SYS, nsc, (int)sizeof(TIN), NA);  // per stage
     double* red = reinterpret_cast<double*>(ring + (size_t)nst * sstride);
-    double* xr = red + (rhs_red ? 2 : 6) * fstride;
+    double* xr = red + 6 * fstride;
     double* pcr = xr + 2 * fstride;  // only when !shuffled
     const int gs = nseg + 2;
     double* tabs = pcr + (shuffled ? 0 : 6 * gs * sub);  // SH: this CTA's factor table
-    double* lanes = tabs + (SH ? tile_tab_doubles(nsc) : 0);  // rhs_red: lane table [k][p]
-    uint64_t* full =
-        reinterpret_cast<uint64_t*>(lanes + (rhs_red ? 32 * TILE_RED_LANE : 0));
+    uint64_t* full = reinterpret_cast<uint64_t*>(tabs + (SH ? tile_tab_doubles(nsc) : 0));
     uint64_t* empty = full + nst;
 
     const int tid = threadIdx.x;
@@ -307,11 +301,6 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         for (int i = threadIdx.x; i < nsc * M * 5; i += blockDim.x) tabs[i] = g0[i];
         const double* g1 = args.gtab + (size_t)args.n_row * 5 + (size_t)c0 * 6;
         for (int i = threadIdx.x; i < nsc * 6; i += blockDim.x) tabs[nsc * M * 5 + i] = g1[i];
-        if (rhs_red) {  // lane-major in global memory, field-major here (no bank conflicts)
-            const double* g2 = args.gtab + tile_red_offset(args.n_row);
-            for (int i = threadIdx.x; i < 32 * TILE_RED_LANE; i += blockDim.x)
-                lanes[(i % TILE_RED_LANE) * 32 + i / TILE_RED_LANE] = g2[i];
-        }
     }
     if (!shuffled && tid < sub) {  // zero guard rows of the PCR buffers
         for (int f = 0; f < 6; ++f) {
@@ -483,17 +472,12 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         if constexpr (SH) {
             const double* sb = tabs + nsc * M * 5 + ql * 6;
             double* w = red + ql * RP + s;
-            if (rhs_red) {  // r0 | r1 only
-                w[0] = sb[0] * (double)db0 - sb[1] * (double)sd;
-                w[fstride] = (double)de[M - 1];
-            } else {
-                w[2 * fstride] = sb[0] * (double)db0 - sb[1] * (double)sd;
-                w[5 * fstride] = (double)de[M - 1];
-                w[0 * fstride] = sb[2];
-                w[1 * fstride] = sb[3];
-                w[3 * fstride] = sb[4];
-                w[4 * fstride] = sb[5];
-            }
+            w[2 * fstride] = sb[0] * (double)db0 - sb[1] * (double)sd;
+            w[5 * fstride] = (double)de[M - 1];
+            w[0 * fstride] = sb[2];
+            w[1 * fstride] = sb[3];
+            w[3 * fstride] = sb[4];
+            w[4 * fstride] = sb[5];
         } else {
             const TC pi_last = -ga[M - 2] * pi;
             const TC r0 = rcp_tc(TC(1) - cb0 * sa);
@@ -512,7 +496,7 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         //   first: l0 xL(p-1) + xF(p) + u0 xL(p) = r0
         //   last:  l1 xF(p) + xL(p) + u1 xF(p+1) = r1
         // One cyclic-reduction level leaves  a xL(p-1) + xL(p) + c xL(p+1) = d.
-        if (shuffled) {
+        if (!CONSTC && shuffled) {  // generated modes: above 32 sub-segments only
             const int per_pass = T / W;  // systems per pass
             const int p = tid % W;
             for (int base = 0; base < sub; base += per_pass) {
@@ -523,19 +507,15 @@ tile_f64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     const int owner = p / nsc;
                     const double* src = red + (p % nsc) * RP + c * sub + sp;
                     if (cl > 1 && owner != c) src = cg::this_cluster().map_shared_rank(src, owner);
-                    r0 = src[(SH ? 0 : 2) * fstride];
-                    r1 = src[(SH ? 1 : 5) * fstride];
-                    if constexpr (!SH) {
-                        l0 = src[0 * fstride];
-                        u0 = src[1 * fstride];
-                        l1 = src[3 * fstride];
-                        u1 = src[4 * fstride];
-                    }
+                    l0 = src[0 * fstride];
+                    u0 = src[1 * fstride];
+                    r0 = src[2 * fstride];
+                    l1 = src[3 * fstride];
+                    u1 = src[4 * fstride];
+                    r1 = src[5 * fstride];
                 }
                 double xf, xl;
-                if constexpr (SH)
-                    reduced_solve_rhs<CYCLIC>(r0, r1, p, nseg, W, lanes + p, 32, xf, xl);
-                else if constexpr (FILT)
+                if constexpr (FILT)
                     reduced_solve_filtered<CYCLIC>(l0, u0, r0, l1, u1, r1, p, nseg, W, filt_r,
                                                    act, xf, xl);
                 else
