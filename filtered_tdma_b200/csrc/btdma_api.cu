@@ -150,12 +150,18 @@ int solve_impl(btdma_t h, const double* A, const double* B, const double* C, con
 
     if (h->method == BTDMA_PASCAL && !(h->flags & BTDMA_FLAG_REFERENCE_ORDER)) {
         // Shapes the narrow kernel does not take and that the segment kernels
-        // would: the wide solve's general form, but for small batches of short
-        // segments, whose shorter sweeps are faster there (B200, P = 4: 512 x 50
-        // 9.5 us against 10.2, 2048 x 50 9.8 / 10.3, 8192 x 50 10.8 / 10.4).
-        const bool general = seg_fits(h, n_sys, n_row, cyclic) &&
-                             !(n_plan % 2 == 0 && n_plan <= 4096 &&
-                               (n_row + h->P - 1) / h->P <= 16);
+        // would: the wide solve's general form, but for small even batches in few
+        // short segments, whose shorter sweeps are faster there as long as the
+        // segments' CTAs are resident together.  B200, us, segment / general:
+        //   P = 2  4096 x 20 7.4 / 9.8     P = 4  4096 x 60 10.5 / 11.1
+        //   P = 6  512 x 90 11.9 / 12.4, 4096 x 90 13.5 / 12.4
+        //   P = 8  512 x 50 12.1 / 10.8, 4096 x 50 23 / 10.8    P = 16  2048 x 250 51 / 11
+        // and periodic
+        //   P = 4  4096 x 60 10.8 / 16.0   P = 6  4096 x 90 13.9 / 15.1
+        //   P = 8  512 x 50 12.8 / 14.8, 4096 x 50 24.9 / 14.9  P = 16  512 x 250 25 / 18
+        const bool few = n_plan % 2 == 0 && n_plan <= 4096 && (n_row + h->P - 1) / h->P <= 16 &&
+                         h->P <= (cyclic ? 8 : 6) && h->P * n_plan <= 6 * 4096;
+        const bool general = seg_fits(h, n_sys, n_row, cyclic) && !few;
         rc = try_tile<double>(A, B, C, D, X, n_sys, n_row, cyclic, h->status, st, false,
                               nullptr, h->tile_shape, 0, false, general, n_plan);
         if (rc < 0) return rc;
