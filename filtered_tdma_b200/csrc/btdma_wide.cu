@@ -8,25 +8,35 @@ struct WidePlan {
     int sys = 0, nsc = 0, cl = 0, nst = 0;
 };
 
-template <int SYS, bool CYCLIC, typename TIN, bool CLUSTER>
+template <int SYS, bool CYCLIC, typename TIN, bool CLUSTER, bool WATCH>
 int launch_wide(const WideMapsGen& maps, const TileArgs& a, const WideGen& gen, cudaStream_t st) {
     const bool odd = sizeof(TIN) == 8 && (a.n_sys & 1) != 0;
-    return launch_tmem<tile_wide_kernel<SYS, CYCLIC, TIN, false, true, CLUSTER>, CLUSTER>(
+    return launch_tmem<tile_wide_kernel<SYS, CYCLIC, TIN, false, true, CLUSTER, WATCH>, CLUSTER>(
         SYS * a.nseg, tile_wide_smem_bytes(SYS, a.nseg, a.nst, (int)sizeof(TIN), odd, a.cl),
         a.cl, a.n_groups, st, maps, a, gen);
 }
 
-template <bool CYCLIC, typename TIN>
+template <bool CYCLIC, typename TIN, bool WATCH>
 int launch_wide_plan(int sys, const WideMapsGen& maps, const TileArgs& a, const WideGen& gen,
                      cudaStream_t st) {
-    if (a.cl > 1) return launch_wide<32, CYCLIC, TIN, true>(maps, a, gen, st);
+    if (a.cl > 1) return launch_wide<32, CYCLIC, TIN, true, WATCH>(maps, a, gen, st);
     switch (sys) {
-        case 256: return launch_wide<256, CYCLIC, TIN, false>(maps, a, gen, st);
-        case 128: return launch_wide<128, CYCLIC, TIN, false>(maps, a, gen, st);
-        case 64: return launch_wide<64, CYCLIC, TIN, false>(maps, a, gen, st);
-        case 16: return launch_wide<16, CYCLIC, TIN, false>(maps, a, gen, st);
-        default: return launch_wide<32, CYCLIC, TIN, false>(maps, a, gen, st);
+        case 256: return launch_wide<256, CYCLIC, TIN, false, WATCH>(maps, a, gen, st);
+        case 128: return launch_wide<128, CYCLIC, TIN, false, WATCH>(maps, a, gen, st);
+        case 64: return launch_wide<64, CYCLIC, TIN, false, WATCH>(maps, a, gen, st);
+        case 16: return launch_wide<16, CYCLIC, TIN, false, WATCH>(maps, a, gen, st);
+        default: return launch_wide<32, CYCLIC, TIN, false, WATCH>(maps, a, gen, st);
     }
+}
+
+// watch: FP64 shapes the narrow kernel does not take.
+template <bool CYCLIC, typename TIN>
+int launch_wide_plan(int sys, const WideMapsGen& maps, const TileArgs& a, const WideGen& gen,
+                     bool watch, cudaStream_t st) {
+    if constexpr (sizeof(TIN) == 8) {
+        if (watch) return launch_wide_plan<CYCLIC, TIN, true>(sys, maps, a, gen, st);
+    }
+    return launch_wide_plan<CYCLIC, TIN, false>(sys, maps, a, gen, st);
 }
 
 // The widest group that fills 512 threads, halved while at most half the SMs have
@@ -157,8 +167,8 @@ int tile_wide_gen(const TIN* A, const TIN* B, const TIN* C, const TIN* D, double
     a.nst = p.nst;
     a.n_groups = (n_sys + p.sys - 1) / p.sys;
     a.status = status;
-    const int rc = cyclic ? launch_wide_plan<true, TIN>(p.sys, maps, a, gen, st)
-                          : launch_wide_plan<false, TIN>(p.sys, maps, a, gen, st);
+    const int rc = cyclic ? launch_wide_plan<true, TIN>(p.sys, maps, a, gen, !narrow, st)
+                          : launch_wide_plan<false, TIN>(p.sys, maps, a, gen, !narrow, st);
     return rc == BTDMA_OK ? 1 : rc;
 }
 

@@ -230,23 +230,23 @@ struct WideFwd {
     double gm2;            // gamma of row M-2
 };
 
-// The reciprocals of a forward pass.  rcp_nr wants normal pivots with normal reciprocals.
-// The form that also serves row counts and batches outside the narrow kernel's keeps the
-// whole FP64 range all the same: PIV_WATCH notes pivots of 2^1017 and more (one above
+// The reciprocals of a forward pass.  rcp_nr wants normal pivots with normal reciprocals,
+// as the narrow kernel's.  Row counts and batches outside that kernel's keep the whole FP64
+// range, as the segment kernels they ran on: PIV_WATCH notes pivots of 2^1017 and more (one above
 // 2^1022 would pass with a reciprocal of 0), subnormal and infinite ones leave NaN, and a
 // warp with such a system takes its rows again from global memory with PIV_EXACT, where
 // that system's lanes use correctly rounded reciprocals.  (B200, 62500 x 250: 110 us
-// unwatched, 113 watched; correctly rounded ones throughout, or a check and a branch a
-// row, 114, and 4 to 7 % over clusters, where the watch costs nothing.)
+// unwatched, 112 watched; correctly rounded ones throughout, or a check and a branch a
+// row, 114, and 4 to 8 % over clusters, where the watch costs at most 1.)
 enum Pivots { PIV_NORMAL = 0, PIV_WATCH = 1, PIV_EXACT = 2 };
 struct PivotWatch {
-    float big = 0.0f;    // PIV_WATCH: NaN once a pivot's high word was, read as a float
+    bool big = false;    // PIV_WATCH: a pivot of 2^1017 or more
     bool exact = false;  // PIV_EXACT: this lane's system needs it
 };
 template <int PIV>
 __device__ __forceinline__ double wide_rcp(double x, PivotWatch& pw) {
     if constexpr (PIV == PIV_WATCH)
-        pw.big = fmaf(__int_as_float(__double2hiint(x)), 0.0f, pw.big);
+        pw.big |= (__double2hiint(x) & 0x7f800000) == 0x7f800000;
     double r = rcp_nr(x);
     if constexpr (PIV == PIV_EXACT) {
         if (pw.exact) r = Exact64::rcp(x);
@@ -256,7 +256,7 @@ __device__ __forceinline__ double wide_rcp(double x, PivotWatch& pw) {
 // Whether a sub-segment's pass met a pivot outside rcp_nr's range (or NaN in the data); d0
 // and dep: the right-hand sides of its row 0, whose chain ends there, and its last row.
 __device__ __forceinline__ bool pivots_out_of_range(const PivotWatch& pw, double d0, double dep) {
-    return isnan(pw.big) || isnan(d0) || isnan(dep);
+    return pw.big || isnan(d0) || isnan(dep);
 }
 // Row k of the forward pass (the expressions of k_tile.cuh's loop, FP64).
 template <int PIV>
@@ -306,21 +306,22 @@ __device__ __forceinline__ void wide_reduced(const WideFwd& f, double* w, int fs
 }
 
 // FILT: Filtered's reduced system (as tile_f64_kernel's FILT; the mode's segment
-// length counts 32-row sub-segments here).
+// length counts 32-row sub-segments here).  WATCH: pivots of the whole FP64 range.
 template <int SYS, bool CYCLIC, typename TIN, bool FILT = false, bool GEN = false,
-          bool CLUSTER = false>
+          bool CLUSTER = false, bool WATCH = false>
 __global__ void __launch_bounds__(TILE_MAX_THREADS, 1)
 tile_wide_kernel(const __grid_constant__ std::conditional_t<GEN, WideMapsGen, WideMaps> maps,
                  const TileArgs args, const WideGen gen) {
     namespace cg = cooperative_groups;
     static_assert(!FILT || !GEN, "Filtered segments are whole sub-segments");
     static_assert(!CLUSTER || GEN, "clusters run the general form");
+    static_assert(!WATCH || (GEN && sizeof(TIN) == 8), "reads FP64 arrays by their pointers");
     constexpr int M = WIDE_M, TR = WIDE_TROWS;
     constexpr int RPS = tile_rps((int)sizeof(TIN));
     constexpr int SPG = M / RPS;  // stages per group
     constexpr int RP = SYS + 1;
     constexpr bool PAD = GEN && !CYCLIC;
-    constexpr int PIV = GEN && sizeof(TIN) == 8 ? PIV_WATCH : PIV_NORMAL;
+    constexpr int PIV = WATCH ? PIV_WATCH : PIV_NORMAL;
     // a closed gate: nothing to do (TILE_MODE_GATE_ZERO: open while *gate == 0); every
     // CTA reads the same word
     if (!GEN && args.gate != nullptr &&
