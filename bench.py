@@ -730,12 +730,12 @@ def main():
             "frac_of_peak": 48 * cells / (ms * 1e-3) / 1e9 / peak,
             # the design's field passes of 16 B: Z sweep reading theta (its
             # right-hand side computed inside the solve) into the Y layout, Y
-            # sweep into the X layout, X sweep into theta (plus the wall planes)
+            # sweep into the X layout, X sweep into theta
             "design_bytes_per_cell": 48,
             "parity": "tests/test_heat.py::test_gpu_step_benched_grid_matches_oracle",
-            # 5 kernels a step (the sweeps' factor tables are built at
-            # create): Z sweep with the right-hand side, Y wall folds, Y sweep,
-            # X wall folds, X sweep
+            # 3 kernels a step (the sweeps' factor tables are built at
+            # create): the Z sweep with the right-hand side, the Y and X sweeps
+            # with their wall terms
             "launches_per_step": 3, "graph": True,
             "finite": bool(torch.isfinite(th).all().item())}
         heat.close()

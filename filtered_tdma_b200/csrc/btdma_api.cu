@@ -55,8 +55,9 @@ int jmax_launch(btdma_t h, const double* D, int n_sys, int n_row, cudaStream_t s
 // exact: the device word jfinal sets when the batch needs the exact reduced
 // solve (null: the reference's behaviour, no fallback)
 int jfinal_launch(btdma_t h, int n_row, int version, unsigned* exact, cudaStream_t st) {
-    jfinal_kernel<<<1, 32 * SEG_MAX_P, 0, st>>>(h->work, h->J, h->rho_row, n_row, h->P, h->eps_constant,
-                                    version, (h->flags & BTDMA_FLAG_J_HOST) ? 1 : 0, exact);
+    jfinal_kernel<<<1, 32 * SEG_MAX_P, 0, st>>>(h->work, h->J, h->rho_row, n_row, h->P,
+                                                h->eps_constant, version,
+                                                (h->flags & BTDMA_FLAG_J_HOST) ? 1 : 0, exact);
     CK(cudaGetLastError());
     return BTDMA_OK;
 }
@@ -379,8 +380,9 @@ int btdma_destroy(btdma_t h) {
 // each gathered from the [n_row][n_sys] host arrays by a 2-D copy into a
 // contiguous [n_row][chunk] device buffer; with two buffer sets, the copy-in
 // of chunk i + 1 (one copy engine), the solve of chunk i and the copy-out of
-// chunk i - 1 (the other copy engine) overlap.  Systems are independent, so a
-// PaScaL chunk solves exactly as in a whole-batch call; a Filtered batch goes
+// chunk i - 1 (the other copy engine) overlap.  Systems are independent, and a
+// PaScaL chunk is cut as in a whole-batch call (solve_impl's n_plan), so it solves
+// exactly as there; a Filtered batch goes
 // through as one chunk, its truncation depth depending on the whole batch's
 // right-hand sides.
 int btdma_solve_host(btdma_t h, const double* hA, const double* hB, const double* hC,

@@ -5,7 +5,7 @@
 // 46-67) and computes J in a single 256-thread block (k_cal_J_rhs_bound, :220-261).
 // Here one bound per row (max of the two) is kept, and J is computed per segment
 // by a grid-wide max reduction (many blocks + atomicMax on the bit patterns of
-// non-negative doubles) followed by a one-warp finalize that also resets the
+// non-negative doubles) followed by a one-block finalize that also resets the
 // accumulators, so consecutive solves (and graph replays) need no memset.
 #pragma once
 

@@ -22,8 +22,8 @@
 //     terms inside their sweeps (k_tile_sh.cuh), so a step is three kernels;
 //   * each sweep stores its solution in the next one's layout: Z ([kk][jj][ii]) in
 //     the Y sweep's [jj][kk][ii], Y in the X sweep's [ii][kk][jj], X in theta.
-// Axes longer than those sweeps take (512 rows) run the kernels below: the
-// right-hand side and the wall terms as passes of their own.
+// Axes longer than those sweeps take (512 rows), and for the right-hand side fields
+// off 16 bytes, run the kernels below: passes of their own.
 #pragma once
 
 #include "btdma_common.cuh"

@@ -1,10 +1,10 @@
 // Channel momentum ADI sweeps (apps/channel_gpu/MomentumSolverGPU.cu:135-220
 // k_build_{x,y,z} + solve + k_scatter_{x,y,z}, called by adi_{z,y,x}_ at
-// :261-313), with the coefficients generated inside the tiled solve (GEN = 3
-// row tables) instead of stored: the build is a gather of the ghosted field
-// into the sweep layout; the z and y sweeps store their solutions straight back
-// into the field (the tiled solve's layout map), the x sweep through a
-// transposing scatter.
+// :261-313), with the coefficients generated from row tables inside the solve
+// (k_tile_sh.cuh; k_tile.cuh's GEN 3 above 512 rows) instead of stored.  What stands
+// here is what a sweep needs outside the fused step: gathers of the ghosted field into
+// the sweep layout, and the Filtered backend's coefficient and scatter kernels.  Every
+// tiled sweep stores its solution straight into its destination.
 //
 // Field: q[i + (nx + 2) * (j + (ny + 2) * k)] (DeviceField.hpp df_idx), interior
 // i = 1..nx, j = 1..ny, k = 1..nz.  Sweep layouts (system index fastest):

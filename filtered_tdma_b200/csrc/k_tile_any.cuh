@@ -9,15 +9,17 @@
 //             rows; each thread copies its own rows (cp.async, 8 bytes) into its
 //             own column of the ring, so neither the row stride nor the row
 //             count has to suit a tensor map (odd n_sys), and no barrier guards
-//             the ring.  (One cp.async.bulk per row piece instead, which wants no
-//             map either, was measured at 50 cycles a piece: 262144 x 512 in 2.9
-//             ms against 1.1 ms.)
+//             the ring: a refill waits for the thread's own loads only.  (One
+//             cp.async.bulk per row piece instead, which wants no map either, was
+//             measured at 50 cycles a piece: 262144 x 512 in 2.9 ms against 1.1 ms.)
 //   cluster   as in k_tile_wide.cuh.
 //
 // Needs NSC <= 16 sub-segments of 3 to 32 rows per CTA, in one CTA a power of two.
 // The TMA form needs an even n_sys and 16-byte aligned arrays.
-// Measured on B200 (us, segment kernels before / now): 65536 x 192 TMA 246 / 99,
-// 48268 x 85 212 / 43, 5000 x 1537 (odd, cp.async) 1163 at 4589 x 512 / 33.
+// Measured on B200 (us, segment kernels / now): TMA 65536 x 192 176 / 105, 48268 x 85
+// 83 / 46, 20000 x 700 818 / 199; cp.async 48269 x 85 141 / 60, 4589 x 1537 3813 / 119
+// (P = 4, and 16 above 250 rows).  Every form spills (248 to 400 bytes of stores at 128
+// registers: run-time lengths keep both ends of every row block alive).
 #pragma once
 
 #include <cooperative_groups.h>
@@ -37,7 +39,7 @@ struct AnyMaps {
 };
 
 struct AnyArgs {
-    const double* in[4];  // A, B, C, D of the cp.async form
+    const double* in[4];  // A, B, C, D (read through them by the cp.async form)
     double* X;
     int n_sys, n_row;
     int sys;       // systems per CTA, a multiple of 16

@@ -17,7 +17,9 @@
 //
 // Measured on B200 (k_tile.cuh's modes before / now): heat sweeps of 256 x 384 x 512, Z
 // 339 / 286 us, Y 279 + 14 (its fold) / 185, X 199 / 140; momentum 256^3 209 / 167 for
-// the three.  Z reads 2.25 cells a cell from L2; X is at 90 % of the copy bandwidth.
+// the three.  Z reads 2.25 cells a cell from L2, and SH_HEAT spills (120 bytes of stores,
+// 156 of loads at 128 registers: both systems' 32 right-hand sides live through the
+// stencil); X is at 90 % of the copy bandwidth.
 // Wider groups alone did nothing for the old modes (X 199 -> 227 us at 32 systems); rows
 // stored with single elements at their misaligned ends took X 250 us; 20 systems a group
 // for the 24 sub-segments of Y (240 threads, 160-byte pieces) 195 us.
@@ -241,8 +243,9 @@ tile_sh_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ S
         if constexpr (MODE == SH_HEAT) {
             // the 7-point right-hand side (the reference's rhs_kernel and build_lhs_z,
             // apps/heat_gpu/solve_theta.cu:121-202), ghosts computed where they are
-            // read: a row is finished when the one above it is read; row 0 takes its lower neighbour in the last stage, row M - 1 its upper
-            // one in the first (from the neighbouring sub-segments' rows)
+            // read: a row is finished when the one above it is read; row 0 takes its
+            // lower neighbour in the last stage, row M - 1 its upper one in the first
+            // (from the neighbouring sub-segments' rows)
             const int ix = args.fblk;
             const double bx = args.bx, by = args.by, bz = args.bz;
             const double diag = 1.0 + (-2.0 * bx) + (-2.0 * by) + (-2.0 * bz);

@@ -1,7 +1,7 @@
 // Wide variant of the register-tiled segmented solve (k_tile.cuh): sub-segments
-// of 32 rows, whose elimination state is held half in registers and half in
-// tensor memory, so a CTA takes twice the systems and every row of a TMA box is
-// twice as wide in HBM.
+// of 32 rows, whose elimination state is held partly in registers (12 rows) and
+// partly in tensor memory (20 rows), so a CTA takes twice the systems and every row
+// of a TMA box is twice as wide in HBM.
 //
 // Why: the DRAM serves a stream of row pieces (SYS x element bytes, rows a full
 // row of the batch apart) at a rate that grows with the piece width: 64-byte
@@ -10,15 +10,16 @@
 // rows in registers (24 bytes a row), which caps it at 16 systems of 512 rows
 // per SM.  The SM's 256 KB of tensor memory is per-thread storage too: a warp
 // reads and writes its own quarter of the lanes (tcgen05.st / tcgen05.ld, 32
-// lanes x 32-bit columns), one 96-column slice per warp holding 16 rows' alpha,
-// gamma and delta of each thread.  With it a CTA takes 32 systems of 512 rows.
+// lanes x 32-bit columns), one 120-column slice per warp holding WIDE_TROWS = 20
+// rows' alpha, gamma and delta of each thread.  With it a CTA takes 32 systems of 512
+// rows.  (16 rows there left 56 to 128 bytes of spills.)
 //
 //   forward   thread (s, q) = system s, rows 32 q .. 32 q + 31: the pass of
-//             k_tile.cuh over 32 rows; after row 15 the state of rows 0..15
-//             moves to tensor memory, rows 16..31 stay in registers.
+//             k_tile.cuh over 32 rows; the state of rows 0..19 moves to tensor
+//             memory four rows at a time, rows 20..31 stay in registers.
 //   reduced   one system per group of W lanes (reduced_solve_shfl), half as
 //             many rows as with 16-row sub-segments.
-//   back      rows 31..16 from registers, then rows 15..0 from tensor memory.
+//   back      rows 31..20 from registers, then rows 19..0 from tensor memory.
 //
 // The ring is that of k_tile.cuh (full / empty mbarriers per stage, refills
 // issued by a rotating producer warp), with unhinted polls.  A, B, C, D are
@@ -27,11 +28,12 @@
 // multiple of 16 bytes and 16-byte aligned arrays; SYS = 16 (NSEG = 16) to 256
 // systems, so that a CTA has 256 to 512 threads.
 //
-// Measured on B200 (262144 x 512): FP64 0.81 ms, FP32 storage 0.52 ms, 102 % and
-// 95 % of the copy bandwidth at the algorithmic 40 / 24 bytes a row (before,
-// with half the rows eliminated a second time from L2: 1.16 / 0.88 ms; the
-// DRAM moved 1.15x the bytes and each row's arithmetic ran 1.5 times).  Bound by
-// DRAM; with 6 / 5 / 4 ring stages of 32 KB it takes 0.811 / 0.815 / 0.857 ms.
+// Measured on B200 (262144 x 512), every pass on another batch: FP64 0.85 ms, FP32
+// storage 0.62 ms, 98 % and 80 % of the copy bandwidth at the algorithmic 40 / 24
+// bytes a row (before, with half the rows eliminated a second time from L2: 1.16 / 0.87
+// ms; the DRAM moved 1.15x the bytes and each row's arithmetic ran 1.5 times).
+// Launched back to back, on one batch or two in turn, 0.81 and 0.53 ms.  Bound by DRAM;
+// with 6 / 5 / 4 ring stages of 32 KB it takes 0.811 / 0.815 / 0.857 ms so.
 #pragma once
 
 #include <cooperative_groups.h>

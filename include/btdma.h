@@ -148,10 +148,11 @@ int btdma_solve_out(btdma_t h, const double* A, const double* B, const double* C
  * works, without overlap).  No reference counterpart: the reference's callers
  * copy to the device themselves (cudaMemcpy) and call solve.  The batch moves
  * in chunks of systems through two device buffer sets that the handle
- * allocates on first use (5 arrays of about n_sys / 8 systems each, kept until
+ * allocates on first use (5 arrays of about n_sys / 16 systems each, kept until
  * btdma_destroy or a larger call): the copy-in of one chunk, the solve of the
  * previous one and the copy-out of the one before overlap on the GPU's two
- * copy engines.  PaScaL chunks solve exactly as a whole-batch btdma_solve_out;
+ * copy engines.  PaScaL chunks solve exactly as a whole-batch btdma_solve_out on
+ * 16-byte aligned arrays;
  * Filtered batches go through as one chunk (their truncation depth depends on
  * the whole batch).  Stream-ordered on `stream`: hX is complete once `stream`
  * reaches this point; successive calls on one handle are serialised.  FP64
@@ -305,7 +306,9 @@ int btdma_ragged_set_plan(btdma_t h, const btdma_ragged_bucket* buckets, int n);
  * coefficients are generated inside the solve (never stored); ix, iy, iz must
  * be multiples of 16.  btdma_heat_step runs n_steps steps, as one captured
  * CUDA graph replayed per step when use_graph != 0 (captured on the first call
- * for this theta pointer).  btdma_heat_init writes the reference's initial
+ * for this theta pointer; not into a stream that is itself capturing, where
+ * use_graph = 0 serves).  theta at 16-byte alignment takes the fused Z sweep,
+ * any other 8-byte one a right-hand-side pass more.  btdma_heat_init writes the reference's initial
  * field; btdma_heat_l2_error returns the reference's global L2 error against
  * the manufactured solution at physical time t_phys (sum over interior cells
  * divided by (ix + 1)(iy + 1)(iz + 1), heat_cpu/main.cpp:59-79; blocking). */
